@@ -93,7 +93,7 @@ struct pann_index {
   int32_t q_offset = 0;
   float q_bound = 1.0f;  // mips: the trimmed bound
   bool graph_borrowed = false;  // d_graph belongs to another index
-  uint32_t gt_fallbacks = 0;  // queries of the last float groundtruth recomputed by the plain kernel
+  pann::DevBuf gt;  // brute-force groundtruth workspace: operand images and candidate buffers (gt_tensor.cu), bounded
   uint32_t starts_cached_n = 0;
   uint32_t starts_cached[64] = {};
 };

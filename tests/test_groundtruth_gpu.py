@@ -1,0 +1,61 @@
+"""Exact top-k on the tensor cores (csrc/gt_tensor.cu) against the plain FP64 / integer kernel, which answers the
+same call with PANN_GT_PLAIN set: ids and distances equal bit for bit (both are exact, ties by id)."""
+import numpy as np
+import pytest
+
+from conftest import has_gpu, random_points
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not has_gpu(), reason="needs a GPU")]
+
+import parlayann_b200 as P  # noqa: E402
+
+# points, queries, dimensions, k: ends of the 128-row tiles, of the 64..256-query blocks, of K's 32-byte steps and
+# 64-byte chunks, of the candidate buffers (64, 256), rows too long for more than 64 queries a block, more k than points
+SHAPES = [(1, 1, 1, 1), (50, 3, 7, 60), (127, 64, 16, 5), (129, 65, 33, 64), (4096, 256, 64, 65), (4097, 257, 65, 10),
+          (20000, 300, 100, 256), (9000, 20, 700, 20), (3000, 10, 40, 257)]
+
+
+def both(base, q, k, metric, monkeypatch):
+    idx = P.Index(base, 4, metric)
+    got = idx.groundtruth(q, k)
+    monkeypatch.setenv("PANN_GT_PLAIN", "1")
+    plain = idx.groundtruth(q, k)
+    monkeypatch.delenv("PANN_GT_PLAIN")
+    np.testing.assert_array_equal(got[0], plain[0])
+    np.testing.assert_array_equal(got[1], plain[1])
+    idx.close()
+    return got
+
+
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+@pytest.mark.parametrize("dtype", [np.uint8, np.int8, np.float32])
+@pytest.mark.parametrize("n,nq,d,k", SHAPES)
+def test_equals_plain_kernel(n, nq, d, k, dtype, metric, lib_built, monkeypatch):
+    both(random_points(dtype, n, d, n + d), random_points(dtype, nq, d, nq + d), k, metric, monkeypatch)
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.int8])
+def test_equal_distances_by_id(dtype, lib_built, monkeypatch):
+    """Few distinct 8-bit points: thousands of equal scores across tiles and slices."""
+    rng = np.random.default_rng(3)
+    both(rng.integers(0, 2, (30000, 5)).astype(dtype), rng.integers(0, 2, (200, 5)).astype(dtype), 70, P.L2, monkeypatch)
+
+
+def test_float_scales(lib_built, monkeypatch):
+    """Values far from 1, one query far from the others, a NaN point (never an answer)."""
+    rng = np.random.default_rng(4)
+    base = rng.standard_normal((6000, 48)).astype(np.float32)
+    q = rng.standard_normal((40, 48)).astype(np.float32)
+    both(base * np.float32(1e8), q * np.float32(1e8), 10, P.L2, monkeypatch)
+    both(base * np.float32(1e-4), q * np.float32(1e-4), 10, P.MIPS, monkeypatch)
+    far = q.copy()
+    far[7] *= np.float32(1e9)
+    both(base, far, 10, P.L2, monkeypatch)
+    nan = np.concatenate([base, base[:1]])
+    nan[-1, 5] = np.nan
+    idx = P.Index(nan, 4)
+    ids, dd = idx.groundtruth(q, 10)
+    idx.close()
+    want = both(base, q, 10, P.L2, monkeypatch)
+    np.testing.assert_array_equal(ids, want[0])
+    np.testing.assert_array_equal(dd, want[1])
