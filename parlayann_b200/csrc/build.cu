@@ -7,10 +7,9 @@
 //                  which is skipped as a neighbour; the visited list is kept)
 //                                                        (index.h:247-264)
 //   2. prune       candidates = visited list + current out-neighbours with
-//                  their distances, sorted by (dist, id) with a segmented
-//                  radix sort, then the greedy alpha-pruning of robustPrune
-//                  (index.h:63-120), written straight into the graph rows
-//                                                        (index.h:265-273)
+//                  their distances, sorted by (dist, id), then the greedy
+//                  alpha-pruning of robustPrune (index.h:63-120; prune.cuh),
+//                  written straight into the graph rows (index.h:265-273)
 //   3. reverse     (new neighbour, inserted point) pairs, stable radix sort by
 //                  neighbour = group_by_key (index.h:281-285); per target,
 //                  append without repeats when it fits, else robustPrune of
@@ -26,6 +25,9 @@
 
 #include "common.cuh"
 #include "index.cuh"
+#include "prune.cuh"
+#include "rowscore.cuh"
+#include "tiers.cuh"
 
 namespace pann {
 
@@ -105,233 +107,62 @@ __global__ void __launch_bounds__(128) assemble_kernel(const uint8_t* __restrict
   }
 }
 
-// Greedy part of robustPrune (index.h:85-116) on a (dist,id)-sorted segment:
-// drop repeated ids, then repeatedly take the first live candidate p* (skipping
-// the point itself) and kill every later p' with alpha * d(p*, p') <= d(p, p')
-// (compared in double). Killed entries get the flag bit; the selection is
-// written to the point's graph row, padded.
-template <int DT, int MT>
-__global__ void __launch_bounds__(128) greedy_prune_kernel(const uint8_t* __restrict__ points, uint64_t stride, int d,
-                                                           int nchunks, uint32_t* graph, uint32_t R, uint32_t njobs,
-                                                           const uint32_t* __restrict__ pts,
-                                                           const uint32_t* __restrict__ seg_begin,
-                                                           const uint32_t* __restrict__ seg_end, uint64_t* keys,
-                                                           double alpha, unsigned long long* dist_cmps) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const unsigned FULL = 0xFFFFFFFFu;
-  uint8_t* qs = smem + (size_t)warp * stride;
-  for (uint32_t job = blockIdx.x * wpb + warp; job < njobs; job += gridDim.x * wpb) {
-    const uint32_t p = pts[job];
-    uint64_t* K = keys + seg_begin[job];
-    const uint32_t m = seg_end[job] - seg_begin[job];
-    // unique by id (:86-88): equal ids carry equal distances, so repeats are adjacent
-    for (uint32_t b = 0; b < m; b += 32) {
-      uint32_t i = b + lane;
-      bool dup = false;
-      if (i < m && i > 0) dup = key_id(K[i]) == key_id(K[i - 1]);
-      __syncwarp();
-      if (dup) K[i] |= PANN_VFLAG;
-    }
-    __syncwarp();
-    uint32_t nsel = 0, idx = 0;
-    unsigned long long cmps = 0;
-    uint32_t* row = graph + (uint64_t)p * R;
-    while (nsel < R && idx < m) {
-      // next live candidate at or after idx
-      int found = -1;
-      for (uint32_t b = idx; b < m && found < 0; b += 32) {
-        uint32_t i = b + lane;
-        bool live = i < m && !(K[i] & PANN_VFLAG);
-        unsigned msk = __ballot_sync(FULL, live);
-        if (msk) found = (int)(b + __ffs(msk) - 1);
-      }
-      if (found < 0) break;
-      const uint32_t pstar = key_id(K[found]);
-      idx = (uint32_t)found + 1;
-      if (pstar == p) continue;  // :99-101
-      if (lane == 0) row[nsel] = pstar;
-      nsel++;
-      stage_query<DT, MT>(qs, points + (uint64_t)pstar * stride, nchunks, lane);
-      __syncwarp();
-      int32_t qq = 0;
-      if (DT != DT_F32 && MT == MT_L2) qq = sq_norm_int<DT>(reinterpret_cast<const uint4*>(qs), nchunks);
-      for (uint32_t b = idx; b < m; b += 32) {
-        uint32_t i = b + lane;
-        bool live = false;
-        uint64_t k = 0;
-        if (i < m) {
-          k = K[i];
-          live = !(k & PANN_VFLAG);
-        }
-        cmps += __popc(__ballot_sync(FULL, live));
-        if (live) {
-          float dsp = point_dist<DT, MT>(points + (uint64_t)key_id(k) * stride, qs, d, nchunks, qq);
-          double dpp = (double)key_dist(k);
-          if (__dmul_rn(alpha, (double)dsp) <= dpp) K[i] = k | PANN_VFLAG;
-        }
-      }
-      __syncwarp();
-    }
-    for (uint32_t j = nsel + lane; j < R; j += 32) row[j] = PANN_PAD;
-    if (lane == 0) atomicAdd(dist_cmps, cmps);
-    __syncwarp();
-  }
-}
-
-// Distance of the row at `row` (shared or global memory: generic loads) to the
-// point staged at qs, with point_dist's arithmetic (common.cuh).
-template <int DT, int MT>
-__device__ __forceinline__ float row_dist_generic(const uint8_t* row, const uint8_t* qs, int nchunks, int32_t qq) {
-  if (DT == DT_F32) {
-    const float4* r = reinterpret_cast<const float4*>(row);
-    const float4* q = reinterpret_cast<const float4*>(qs);
-    float acc = 0.0f;
-    for (int c0 = 0; c0 < nchunks; c0 += ROW_CHUNKS) {
-      float4 b[ROW_CHUNKS];
-#pragma unroll
-      for (int c = 0; c < ROW_CHUNKS; c++)
-        if (c0 + c < nchunks) b[c] = r[c0 + c];
-#pragma unroll
-      for (int c = 0; c < ROW_CHUNKS; c++)
-        if (c0 + c < nchunks) acc = f32_chunk<MT>(acc, b[c], q[c0 + c]);
-    }
-    return MT == MT_L2 ? acc : -acc;
-  } else {
-    const uint4* r = reinterpret_cast<const uint4*>(row);
-    const uint4* q = reinterpret_cast<const uint4*>(qs);
-    int32_t pq = 0, pp = 0;
-    for (int c = 0; c < nchunks; c++) int_chunk<DT, MT>(r[c], q[c], pq, pp);
-    return int_result<MT>(qq, pq, pp);
-  }
-}
-
-// The greedy part of robustPrune as greedy_prune_kernel computes it, with one
-// block of 128 threads per job and the candidates' rows staged in shared
-// memory (the first `cap_rows` of the segment; later ones are read from
-// global memory): each selection is one pass of the block over the live
-// candidates after it, every distance from shared memory, instead of a
-// warp's dependent global loads. Same answers: the same candidates, the same
-// order of selections, the same float / integer distance and the alpha test
-// in double.
-template <int DT, int MT>
-__global__ void __launch_bounds__(128) greedy_prune_block_kernel(const uint8_t* __restrict__ points, uint64_t stride,
-                                                                 int nchunks, uint32_t* graph, uint32_t R,
-                                                                 uint32_t njobs, const uint32_t* __restrict__ pts,
-                                                                 const uint32_t* __restrict__ seg_begin,
-                                                                 const uint32_t* __restrict__ seg_end, uint64_t* keys,
-                                                                 double alpha, uint32_t cap_rows,
-                                                                 unsigned long long* dist_cmps) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint8_t* qs = smem;                     // p*
-  uint8_t* rows = smem + stride;          // cap_rows staged candidate rows
-  __shared__ int s_found;
-  __shared__ unsigned long long s_cmps;
-  for (uint32_t job = blockIdx.x; job < njobs; job += gridDim.x) {
-    const uint32_t p = pts[job];
-    uint64_t* K = keys + seg_begin[job];
-    const uint32_t m = seg_end[job] - seg_begin[job];
-    const uint32_t staged = m < cap_rows ? m : cap_rows;
-    // unique by id (index.h:86-88), and the rows of the first `staged` candidates
-    for (uint32_t i = tid; i < m; i += 128)
-      if (i > 0 && key_id(K[i]) == key_id(K[i - 1])) K[i] |= PANN_VFLAG;
-    for (uint32_t x = tid; x < staged * (uint32_t)nchunks; x += 128) {
-      const uint32_t r = x / nchunks, c = x - r * nchunks;
-      reinterpret_cast<uint4*>(rows + (size_t)r * stride)[c] =
-          __ldg(reinterpret_cast<const uint4*>(points + (uint64_t)key_id(K[r]) * stride) + c);
-    }
-    if (tid == 0) s_cmps = 0;
-    __syncthreads();
-    uint32_t nsel = 0, idx = 0;
-    uint32_t* row = graph + (uint64_t)p * R;
-    while (nsel < R && idx < m) {
-      if (warp == 0) {
-        int found = -1;
-        for (uint32_t b = idx; b < m && found < 0; b += 32) {
-          const uint32_t i = b + lane;
-          const bool live = i < m && !(K[i] & PANN_VFLAG);
-          const unsigned msk = __ballot_sync(0xFFFFFFFFu, live);
-          if (msk) found = (int)(b + __ffs(msk) - 1);
-        }
-        if (lane == 0) s_found = found;
-      }
-      __syncthreads();
-      const int found = s_found;
-      if (found < 0) break;
-      const uint32_t pstar = key_id(K[found]);
-      idx = (uint32_t)found + 1;
-      if (pstar == p) {  // :99-101
-        __syncthreads();
-        continue;
-      }
-      if (tid == 0) row[nsel] = pstar;
-      nsel++;
-      const uint8_t* src = (uint32_t)found < staged ? rows + (size_t)found * stride : points + (uint64_t)pstar * stride;
-      for (int c = tid; c < nchunks; c += 128) {
-        uint4 v = reinterpret_cast<const uint4*>(src)[c];
-        // staged as stage_query stages it: float32 Euclidean rows negated (f32_chunk forms x + (-q))
-        if (DT == DT_F32 && MT == MT_L2) v = make_uint4(v.x ^ 0x80000000u, v.y ^ 0x80000000u, v.z ^ 0x80000000u, v.w ^ 0x80000000u);
-        reinterpret_cast<uint4*>(qs)[c] = v;
-      }
-      __syncthreads();
-      int32_t qq = 0;
-      if (DT != DT_F32 && MT == MT_L2) qq = sq_norm_int<DT>(reinterpret_cast<const uint4*>(qs), nchunks);
-      uint32_t my_cmps = 0;
-      for (uint32_t i = idx + tid; i < m; i += 128) {
-        const uint64_t k = K[i];
-        if (k & PANN_VFLAG) continue;
-        my_cmps++;
-        const uint8_t* r = i < staged ? rows + (size_t)i * stride : points + (uint64_t)key_id(k) * stride;
-        const float dsp = row_dist_generic<DT, MT>(r, qs, nchunks, qq);
-        if (__dmul_rn(alpha, (double)dsp) <= (double)key_dist(k)) K[i] = k | PANN_VFLAG;
-      }
-      for (int o = 16; o; o >>= 1) my_cmps += __shfl_xor_sync(0xFFFFFFFFu, my_cmps, o);
-      if (lane == 0 && my_cmps) atomicAdd(&s_cmps, (unsigned long long)my_cmps);
-      __syncthreads();
-    }
-    for (uint32_t j = nsel + tid; j < R; j += 128) row[j] = PANN_PAD;
-    __syncthreads();
-    if (tid == 0) atomicAdd(dist_cmps, s_cmps);
-  }
-}
-
-// Reverse-edge pairs: key = new neighbour (PAD for empty slots), value = inserted point.
+// Reverse-edge pairs: key = new neighbour (n for empty slots, so that the sort
+// needs only n's bits), value = inserted point.
 __global__ void reverse_pairs_kernel(const uint32_t* __restrict__ graph, uint32_t R, const uint32_t* __restrict__ pts,
-                                     uint32_t B, uint32_t* kout, uint32_t* vout) {
+                                     uint32_t B, uint32_t n, uint32_t* kout, uint32_t* vout) {
   uint64_t total = (uint64_t)B * R;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t i = (uint32_t)(t / R), j = (uint32_t)(t - (uint64_t)i * R);
     uint32_t p = pts[i];
-    kout[t] = graph[(uint64_t)p * R + j];
+    kout[t] = min(graph[(uint64_t)p * R + j], n);
     vout[t] = p;
   }
 }
 
 // Per group (target j with m new in-edges): append without repeats when
 // m + deg(j) <= R (add_neighbors_without_repeats, index.h:140-146,294-297),
-// else record a robustPrune job (index.h:298-301). One warp per group.
-__global__ void reverse_classify_kernel(uint32_t* graph, uint32_t R, const uint32_t* __restrict__ uniq,
-                                        const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offs,
-                                        const uint32_t* __restrict__ num_runs, const uint32_t* __restrict__ vals,
-                                        uint32_t* job_pts, uint32_t* job_off, uint32_t* job_n, uint32_t* job_begin,
-                                        uint32_t* njobs, unsigned long long* seg_total) {
+// else a robustPrune job (index.h:298-301) of one of four classes:
+//   0 few fresh candidates (the new ones and the row's entries since its last
+//     prune): their distance table fits reprune_kernel's dcap
+//   1 up to cap1 candidates: prune_lazy_kernel, a warp per job
+//   2 up to cap2: prune_block_kernel, a block per job
+//   3 more: assembled and sorted in global memory first
+// Classes 0 and 1 share one job array, filled from its two ends (jobs_cap
+// entries); classes 2 and 3 have big_cap entries each. One warp per group.
+struct ClassifyArgs {
+  uint32_t* graph;
+  uint32_t R, n;
+  uint32_t* nclean;
+  const uint32_t *uniq, *counts, *offs, *num_runs, *vals;
+  uint32_t *job_pts, *job_off, *job_n;  // classes 0 and 1
+  uint32_t jobs_cap;
+  uint32_t *big_pts, *big_off, *big_n;  // classes 2, then 3 at big_cap
+  uint32_t big_cap;
+  uint32_t* big_begin;                  // class 3: segment starts
+  uint32_t* njobs;                      // four counts
+  unsigned long long *seg_total, *cands_total;
+  uint32_t cap0, dcap, cap1, cap2;
+};
+__global__ void reverse_classify_kernel(ClassifyArgs a) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
-  const uint32_t runs = *num_runs;
+  const uint32_t runs = *a.num_runs;
+  const uint32_t R = a.R;
   for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < runs; r += (gridDim.x * blockDim.x) >> 5) {
-    const uint32_t tgt = uniq[r];
-    if (tgt == PANN_PAD) continue;
-    const uint32_t m = counts[r], off = offs[r];
-    uint32_t* row = graph + (uint64_t)tgt * R;
+    const uint32_t tgt = a.uniq[r];
+    if (tgt >= a.n) continue;
+    const uint32_t m = a.counts[r], off = a.offs[r];
+    uint32_t* row = a.graph + (uint64_t)tgt * R;
     uint32_t deg = 0;
     for (uint32_t b = 0; b < R; b += 32) {
       uint32_t j = b + lane;
       deg += __popc(__ballot_sync(FULL, j < R && row[j] != PANN_PAD));
     }
+    const uint32_t clean = min(deg, a.nclean[tgt]);
     if (m + deg <= R) {
       // old neighbours not among the new candidates, in order
-      uint32_t keep_cnt = 0;
+      uint32_t keep_cnt = 0, kept_clean = 0;
       uint32_t oldv[32];  // up to 1024 / 32 per lane
       bool keepv[32];
       int nslot = (int)((R + 31) / 32);
@@ -341,26 +172,40 @@ __global__ void reverse_classify_kernel(uint32_t* graph, uint32_t R, const uint3
         bool keep = v != PANN_PAD;
         if (keep)
           for (uint32_t t = 0; t < m; t++)
-            if (vals[off + t] == v) { keep = false; break; }
+            if (a.vals[off + t] == v) { keep = false; break; }
         oldv[s] = v;
         keepv[s] = keep;
+        kept_clean += __popc(__ballot_sync(FULL, keep && j >= deg - clean));
       }
       __syncwarp();
-      for (uint32_t t = lane; t < m; t += 32) row[t] = vals[off + t];
+      for (uint32_t t = lane; t < m; t += 32) row[t] = a.vals[off + t];
       for (int s = 0; s < nslot; s++) {
         unsigned msk = __ballot_sync(FULL, keepv[s]);
         if (keepv[s]) row[m + keep_cnt + __popc(msk & ((1u << lane) - 1))] = oldv[s];
         keep_cnt += __popc(msk);
       }
       for (uint32_t j = m + keep_cnt + lane; j < R; j += 32) row[j] = PANN_PAD;
+      if (lane == 0) a.nclean[tgt] = kept_clean;
       __syncwarp();
     } else if (lane == 0) {
-      // a segment of exactly m candidates + deg current neighbours, packed by an atomic cursor
-      uint32_t t = atomicAdd(njobs, 1u);
-      job_pts[t] = tgt;
-      job_off[t] = off;
-      job_n[t] = m;
-      job_begin[t] = (uint32_t)atomicAdd(seg_total, (unsigned long long)(m + deg));
+      const uint32_t tot = m + deg;
+      const uint64_t table = (uint64_t)(tot - clean) * tot;
+      const int c = tot <= a.cap0 && table <= a.dcap ? 0 : tot <= a.cap1 ? 1 : tot <= a.cap2 ? 2 : 3;
+      const uint32_t t = atomicAdd(a.njobs + c, 1u);
+      atomicAdd(a.cands_total, (unsigned long long)tot);
+      if (c < 2) {
+        const uint32_t at = c == 0 ? t : a.jobs_cap - 1 - t;
+        a.job_pts[at] = tgt;
+        a.job_off[at] = off;
+        a.job_n[at] = m;
+      } else {
+        const uint32_t at = c == 2 ? t : a.big_cap + t;
+        a.big_pts[at] = tgt;
+        a.big_off[at] = off;
+        a.big_n[at] = m;
+        // a segment of exactly m candidates + deg current neighbours, packed by an atomic cursor
+        if (c == 3) a.big_begin[t] = (uint32_t)atomicAdd(a.seg_total, (unsigned long long)tot);
+      }
     }
   }
 }
@@ -371,8 +216,10 @@ __global__ void __launch_bounds__(128) sort_neighbors_kernel(const uint8_t* __re
                                                              int nchunks, uint32_t* graph, uint32_t R, uint64_t n) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  uint8_t* qs = smem + (size_t)warp * (stride + 16ull * R);
-  uint64_t* kin = reinterpret_cast<uint64_t*>(qs + stride);
+  constexpr uint32_t SCR = row_score_scratch<DT>();
+  uint8_t* qs = smem + (size_t)warp * (stride + SCR + 16ull * R);
+  uint8_t* stg = qs + stride;
+  uint64_t* kin = reinterpret_cast<uint64_t*>(stg + SCR);
   uint64_t* kout = kin + R;
   for (uint64_t v = (uint64_t)blockIdx.x * wpb + warp; v < n; v += (uint64_t)gridDim.x * wpb) {
     stage_query<DT, MT>(qs, points + v * stride, nchunks, lane);
@@ -381,17 +228,14 @@ __global__ void __launch_bounds__(128) sort_neighbors_kernel(const uint8_t* __re
     if (DT != DT_F32 && MT == MT_L2) qq = sq_norm_int<DT>(reinterpret_cast<const uint4*>(qs), nchunks);
     uint32_t* row = graph + v * R;
     uint32_t deg = 0;
-    for (uint32_t b = 0; b < R; b += 32) {
-      uint32_t j = b + lane;
-      uint32_t u = j < R ? row[j] : PANN_PAD;
-      bool ok = u != PANN_PAD;
-      unsigned msk = __ballot_sync(0xFFFFFFFFu, ok);
-      // Points[i].distance(Points[j]): row i is `this`
-      if (ok) {
-        // distance(row v, point u): the query operand is u, the row operand is v
-        float dd = point_dist<DT, MT>(points + (uint64_t)u * stride, qs, d, nchunks, qq);
-        kin[b + __popc(msk & ((1u << lane) - 1))] = make_key(dd, u);
-      }
+    for (uint32_t b = 0; b < R; b += 32) {  // a row's live entries are a prefix
+      const uint32_t j = b + lane;
+      const uint32_t u = j < R ? row[j] : PANN_PAD;
+      const unsigned msk = __ballot_sync(0xFFFFFFFFu, u != PANN_PAD);
+      if (!msk) break;
+      // Points[i].distance(Points[j]): the same float whichever of the two is the staged operand
+      const float dd = warp_score_rows<DT, MT>(points, stride, nchunks, u, __popc(msk), qs, stg, qq, lane);
+      if (u != PANN_PAD) kin[j] = make_key(dd, u);
       deg += __popc(msk);
     }
     __syncwarp();
@@ -432,16 +276,9 @@ static void batch_schedule(uint64_t n, uint64_t m, std::vector<uint64_t>& fl, st
   }
 }
 
-// Which greedy kernel a prune step runs: one warp per job (the default), or
-// one block per job with the candidates' rows staged in shared memory
-// (PANN_PRUNE_KERNEL=block). Measured on the 1M x 96 float build (R 64, L 128,
-// two passes), the block kernel is slower in both steps: 0.91 s against
-// 0.69 s for the insertion prunes, whose lists are the visited nodes, and
-// more for the re-prunes, whose lists are a full row plus its new reverse
-// edges; with 64 KB of staged rows a block, far fewer jobs are resident at
-// once. Both give the same graph.
-static bool prune_block_kernel(bool reprune) {
-  (void)reprune;
+// PANN_PRUNE_KERNEL=block: every prune on prune_block_kernel, a block per job
+// (the class of jobs with many candidates; the same graph).
+static bool prune_all_blocks() {
   static const bool block = [] {
     const char* e = std::getenv("PANN_PRUNE_KERNEL");
     return e && !std::strcmp(e, "block");
@@ -449,37 +286,54 @@ static bool prune_block_kernel(bool reprune) {
   return block;
 }
 
-// robustPrune's greedy part for njobs segments: the block kernel with up to
-// 64 KB of staged candidate rows per block, or the warp-per-job kernel.
+// Blocks of a grid that fills the device once, at most `want`.
+template <typename K>
+static int fill_grid(const pann_index* idx, K k, int threads, size_t smem, uint64_t want) {
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smem) != cudaSuccess || occ <= 0) occ = 1;
+  return (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)occ * idx->sm_count));
+}
+
+// Warps per block of a warp-per-job kernel needing `per_warp` shared bytes a warp; 0 if not even one fits.
+static int prune_wpb(const pann_index* idx, size_t per_warp) {
+  for (int w = 4; w >= 1; w >>= 1)
+    if (per_warp * w <= idx->smem_optin) return w;
+  return 0;
+}
+
 template <int DT, int MT>
-static cudaError_t launch_greedy(const pann_index* idx, uint32_t njobs, const uint32_t* pts, const uint32_t* sb,
-                                 const uint32_t* se, uint64_t* keys, double alpha, unsigned long long* cmps,
-                                 bool reprune, cudaStream_t st) {
-  if (njobs == 0) return cudaSuccess;
-  if (!prune_block_kernel(reprune)) {
-    const int wpb = 4;
-    const int blocks = (int)std::min<uint32_t>((njobs + wpb - 1) / wpb, 65535);
-    greedy_prune_kernel<DT, MT><<<blocks, 32 * wpb, wpb * idx->stride, st>>>(
-        idx->d_points, idx->stride, (int)idx->d, (int)idx->nchunks, idx->d_graph, idx->R, njobs, pts, sb, se, keys,
-        alpha, cmps);
-    return cudaGetLastError();
-  }
-  auto k = greedy_prune_block_kernel<DT, MT>;
-  // dynamic + static shared memory must stay within the opt-in limit; rows
-  // past the staged ones are read from global memory (cap_rows may be 0)
-  cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, k);
+static cudaError_t launch_lazy(const pann_index* idx, const PruneArgs& a, uint64_t max_jobs, cudaStream_t st) {
+  auto k = prune_lazy_kernel<DT, MT>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
   if (e != cudaSuccess) return e;
-  const uint64_t limit = (uint64_t)smem_attr_max() - fa.sharedSizeBytes;
-  if (idx->stride > limit) return cudaErrorInvalidValue;
-  const uint32_t cap_rows =
-      (uint32_t)std::min<uint64_t>((64ull << 10) / idx->stride, (limit - idx->stride) / idx->stride);
-  const size_t smem = idx->stride * (1 + (size_t)cap_rows);
-  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t pw = prune_warp_bytes(idx->stride, a.cap, row_score_scratch<DT>());
+  const int wpb = prune_wpb(idx, pw);
+  if (wpb == 0) return cudaErrorInvalidValue;
+  k<<<fill_grid(idx, k, 32 * wpb, pw * wpb, (max_jobs + wpb - 1) / wpb), 32 * wpb, pw * wpb, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int DT, int MT>
+static cudaError_t launch_reprune(const pann_index* idx, const PruneArgs& a, uint64_t max_jobs, cudaStream_t st) {
+  auto k = reprune_kernel<DT, MT>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
   if (e != cudaSuccess) return e;
-  const int blocks = (int)std::min<uint32_t>(njobs, 2u * 65535u);
-  k<<<blocks, 128, smem, st>>>(idx->d_points, idx->stride, (int)idx->nchunks, idx->d_graph, idx->R, njobs, pts, sb, se,
-                               keys, alpha, cap_rows, cmps);
+  const size_t pw = prune_warp_bytes(idx->stride, a.cap, row_score_scratch<DT>()) + 4ull * a.dcap;
+  const int wpb = prune_wpb(idx, pw);
+  if (wpb == 0) return cudaErrorInvalidValue;
+  k<<<fill_grid(idx, k, 32 * wpb, pw * wpb, (max_jobs + wpb - 1) / wpb), 32 * wpb, pw * wpb, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int DT, int MT, bool GATHERED>
+static cudaError_t launch_block(const pann_index* idx, const PruneArgs& a, const PruneSegs& sg, uint64_t max_jobs,
+                                cudaStream_t st) {
+  auto k = prune_block_kernel<DT, MT, GATHERED>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max() - 256);
+  if (e != cudaSuccess) return e;
+  const size_t sm = prune_block_bytes(idx->stride, GATHERED ? 0 : a.cap, row_score_scratch<DT>());
+  if (sm > (size_t)smem_attr_max() - 256) return cudaErrorInvalidValue;
+  k<<<fill_grid(idx, k, PRUNE_BLOCK, sm, max_jobs), PRUNE_BLOCK, sm, st>>>(a, sg);
   return cudaGetLastError();
 }
 
@@ -494,14 +348,14 @@ static cudaError_t dispatch_dm(int dtype, int metric, F&& f) {
   return cudaErrorInvalidValue;
 }
 
+// Device memory of one build: the fixed arrays carved out of one allocation
+// (23 allocations cost milliseconds, and on a busy host far more), the visited
+// lists (regrown if a search visits more), and the segment buffers of the rare
+// prunes that are sorted in global memory.
 struct BuildBufs {
-  DevBuf perm, vis_keys, vis_n, cmps, status, seg_a, seg_b, seg_begin, seg_end, pk_a, pk_b, pv_a, pv_b, uniq, counts,
-      offs, nruns, jobs, job_off, job_n, cub_tmp, counters, start;
+  DevBuf fixed, vis_keys, seg_a, seg_b, seg_tmp, seg_se;
   void release() {
-    for (DevBuf* b : {&perm, &vis_keys, &vis_n, &cmps, &status, &seg_a, &seg_b, &seg_begin, &seg_end, &pk_a, &pk_b,
-                      &pv_a, &pv_b, &uniq, &counts, &offs, &nruns, &jobs, &job_off, &job_n, &cub_tmp, &counters,
-                      &start})
-      b->release();
+    for (DevBuf* b : {&fixed, &vis_keys, &seg_a, &seg_b, &seg_tmp, &seg_se}) b->release();
   }
 };
 
@@ -515,33 +369,41 @@ __global__ void status_or_kernel(const uint32_t* status, uint32_t n, uint32_t* o
   for (int o = 16; o; o >>= 1) acc |= __shfl_xor_sync(0xFFFFFFFFu, acc, o);
   if ((threadIdx.x & 31) == 0 && acc) atomicOr(out, acc);
 }
-__global__ void count_flag_kernel(const uint32_t* status, uint32_t n, uint32_t flag, uint32_t* out) {
-  uint32_t acc = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    acc += (status[i] & flag) ? 1u : 0u;
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
+// One batch's search counters: queries whose status has `flag`, comparisons (into c64[0] and c64[3]) and visits (c64[1]).
+__global__ void batch_sums_kernel(const uint32_t* status, uint32_t flag, const uint32_t* cmps, const uint32_t* vis,
+                                  uint32_t n, uint32_t* flagged, unsigned long long* c64) {
+  unsigned long long c = 0, v = 0;
+  uint32_t f = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    f += (status[i] & flag) ? 1u : 0u;
+    c += cmps[i];
+    v += vis[i];
+  }
+  for (int o = 16; o; o >>= 1) {
+    f += __shfl_xor_sync(0xFFFFFFFFu, f, o);
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (f) atomicAdd(flagged, f);
+    if (c) { atomicAdd(c64, c); atomicAdd(c64 + 3, c); }
+    if (v) atomicAdd(c64 + 1, v);
+  }
 }
-// Sum of end[i] - begin[i] (segment lengths) and of the live degrees of the rows rows[i].
+// Sum of end[i] - begin[i] (segment lengths).
 __global__ void seg_len_sum_kernel(const uint32_t* begin, const uint32_t* end, uint32_t n, unsigned long long* out) {
   unsigned long long acc = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc += end[i] - begin[i];
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
 }
+// Live degrees of the rows rows[i], summed.
 __global__ void degree_sum_kernel(const uint32_t* graph, uint32_t R, const uint32_t* rows, uint32_t n,
                                   unsigned long long* out) {
   unsigned long long acc = 0;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < (uint64_t)n * R;
        e += (uint64_t)gridDim.x * blockDim.x)
     acc += graph[(uint64_t)rows[e / R] * R + e % R] != PANN_PAD;
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
-}
-
-__global__ void sum_kernel(const uint32_t* v, uint32_t n, unsigned long long* out) {
-  unsigned long long acc = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc += v[i];
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
 }
@@ -581,108 +443,166 @@ extern "C" int pann_build(pann_index* idx, const pann_build_params* bp, const ui
 
   // empty graph (Graph(maxDeg, n) is zeroed: every degree 0)
   BCUDA(cudaMemsetAsync(idx->d_graph, 0xFF, sizeof(uint32_t) * R * n, st));
-  // insertion order
-  BCUDA(bb.perm.ensure(4 * n));
-  uint32_t* d_perm = bb.perm.as<uint32_t>();
-  if (perm) {
-    BCUDA(cudaMemcpyAsync(d_perm, perm, 4 * n, cudaMemcpyHostToDevice, st));
-  } else {
-    DevBuf k1, k2, i1;
-    BCUDA(k1.ensure(8 * n)); BCUDA(k2.ensure(8 * n)); BCUDA(i1.ensure(4 * n));
-    perm_keys_kernel<<<(int)std::min<uint64_t>((n + 255) / 256, 65535), 256, 0, st>>>(k1.as<uint64_t>(),
-                                                                                      i1.as<uint32_t>(), n, bp->perm_seed);
-    size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, k1.as<uint64_t>(), k2.as<uint64_t>(), i1.as<uint32_t>(), d_perm,
-                                    (int)n, 0, 64, st);
-    DevBuf tmp;
-    BCUDA(tmp.ensure(tb + 16));
-    BCUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k1.as<uint64_t>(), k2.as<uint64_t>(), i1.as<uint32_t>(), d_perm,
-                                          (int)n, 0, 64, st));
-    BCUDA(cudaStreamSynchronize(st));
-    k1.release(); k2.release(); i1.release(); tmp.release();
-  }
 
   std::vector<uint64_t> fl, ce;
   batch_schedule(n, n, fl, ce);
   uint64_t maxB = 0;
   for (size_t b = 0; b < fl.size(); b++) maxB = std::max(maxB, ce[b] - fl[b]);
-
-  uint32_t vis_cap = std::max<uint32_t>(2 * bp->L + 64, 128);
-  const uint32_t start0 = 0;
-  BCUDA(bb.start.ensure(16));
-  BCUDA(cudaMemcpyAsync(bb.start.p, &start0, 4, cudaMemcpyHostToDevice, st));
-  BCUDA(bb.counters.ensure(256));
-  uint32_t* c32 = bb.counters.as<uint32_t>();  // [0] status or, [1] njobs, [2] flagged count
-  // [0] dist cmps, [1] visited, [2] reverse prune segment cursor, [3] search cmps,
-  // [4] insertion prune candidates, [5] reverse-edge pairs
-  unsigned long long* c64 = reinterpret_cast<unsigned long long*>(c32 + 8);
-  BCUDA(cudaMemsetAsync(bb.counters.p, 0, 256, st));
-
   const uint64_t pairs_cap = maxB * R;
-  auto alloc_batch = [&](uint32_t vcap) -> int {
-    uint64_t segcap = vcap + R;
-    uint64_t seg_items = maxB * segcap;
-    BCUDA(bb.vis_keys.ensure(8 * maxB * vcap));
-    BCUDA(bb.vis_n.ensure(4 * maxB));
-    BCUDA(bb.cmps.ensure(4 * maxB));
-    BCUDA(bb.status.ensure(4 * maxB));
-    BCUDA(bb.seg_a.ensure(8 * seg_items));
-    BCUDA(bb.seg_b.ensure(8 * seg_items));
-    BCUDA(bb.seg_begin.ensure(4 * std::max<uint64_t>(maxB, pairs_cap)));
-    BCUDA(bb.seg_end.ensure(4 * std::max<uint64_t>(maxB, pairs_cap)));
-    BCUDA(bb.pk_a.ensure(4 * pairs_cap)); BCUDA(bb.pk_b.ensure(4 * pairs_cap));
-    BCUDA(bb.pv_a.ensure(4 * pairs_cap)); BCUDA(bb.pv_b.ensure(4 * pairs_cap));
-    BCUDA(bb.uniq.ensure(4 * pairs_cap)); BCUDA(bb.counts.ensure(4 * pairs_cap)); BCUDA(bb.offs.ensure(4 * pairs_cap));
-    BCUDA(bb.nruns.ensure(16));
-    BCUDA(bb.jobs.ensure(4 * pairs_cap)); BCUDA(bb.job_off.ensure(4 * pairs_cap)); BCUDA(bb.job_n.ensure(4 * pairs_cap));
-    // CUB temporary storage: the largest of the three uses
-    size_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;
-    cub::DeviceSegmentedSort::SortKeys(nullptr, t1, bb.seg_a.as<uint64_t>(), bb.seg_b.as<uint64_t>(), (int)seg_items,
-                                       (int)std::max<uint64_t>(maxB, pairs_cap), bb.seg_begin.as<uint32_t>(),
-                                       bb.seg_end.as<uint32_t>(), st);
-    cub::DeviceRadixSort::SortPairs(nullptr, t2, bb.pk_a.as<uint32_t>(), bb.pk_b.as<uint32_t>(), bb.pv_a.as<uint32_t>(),
-                                    bb.pv_b.as<uint32_t>(), (int)pairs_cap, 0, 32, st);
-    cub::DeviceRunLengthEncode::Encode(nullptr, t3, bb.pk_b.as<uint32_t>(), bb.uniq.as<uint32_t>(),
-                                       bb.counts.as<uint32_t>(), bb.nruns.as<uint32_t>(), (int)pairs_cap, st);
-    cub::DeviceScan::ExclusiveSum(nullptr, t4, bb.counts.as<uint32_t>(), bb.offs.as<uint32_t>(), (int)pairs_cap, st);
-    BCUDA(bb.cub_tmp.ensure(std::max(std::max(t1, t2), std::max(t3, t4)) + 256));
-    return PANN_OK;
-  };
-  {
-    int rc = alloc_batch(vis_cap);
-    if (rc) return rc;
-  }
-
+  uint32_t vis_cap = std::max<uint32_t>(2 * bp->L + 64, 128);
   const int dtype = idx->dtype, metric = idx->metric;
   const uint64_t stride = idx->stride;
   const int d = (int)idx->d, nch = (int)idx->nchunks;
   const int wpb = 4;
-  const size_t warp_smem = stride;
+  const uint32_t scratch = row_score_scratch_rt(dtype);
+
+  // Classes of the reverse-edge prunes (ClassifyArgs). The distance table of
+  // class 0 is 6 KB a warp (R 64: 20 fresh candidates), which leaves 12 warps
+  // an SM; class 1 ends at three rows' worth of candidates, where one warp
+  // starts to outlast the rest of the batch.
+  const bool blocks_only = prune_all_blocks();
+  const uint32_t cap0 = (R + 32 + 3) & ~3u, dcap = 1536;
+  uint32_t cap1 = std::max<uint32_t>(3 * R, 192), cap2 = 4096;
+  while (cap2 > 64 && prune_block_bytes(stride, cap2, scratch) > (size_t)smem_attr_max() - 256) cap2 >>= 1;
+  const bool reprune_ok = !blocks_only && prune_wpb(idx, prune_warp_bytes(stride, cap0, scratch) + 4ull * dcap) > 0;
+  const bool lazy_ok = !blocks_only && prune_wpb(idx, prune_warp_bytes(stride, cap1, scratch)) > 0;
+  if (!lazy_ok) cap1 = 0;
+  const uint64_t big_cap = lazy_ok ? pairs_cap / 64 + 16 : pairs_cap;
+
+  // sorts and scans of the reverse edges: keys are point ids and n
+  int key_bits = 1;
+  while (key_bits < 32 && (1ull << key_bits) <= n) key_bits++;
+  size_t cub_bytes = 0;
+  {
+    size_t t[4] = {0, 0, 0, 0};
+    uint32_t* u = nullptr;
+    cub::DeviceRadixSort::SortPairs(nullptr, t[0], u, u, u, u, (int)pairs_cap, 0, key_bits, st);
+    cub::DeviceRunLengthEncode::Encode(nullptr, t[1], u, u, u, u, (int)pairs_cap, st);
+    cub::DeviceScan::ExclusiveSum(nullptr, t[2], u, u, (int)pairs_cap, st);
+    uint64_t* k = nullptr;
+    if (!perm) cub::DeviceRadixSort::SortPairs(nullptr, t[3], k, k, u, u, (int)n, 0, 64, st);
+    cub_bytes = *std::max_element(t, t + 4) + 256;
+  }
+  size_t fixed_bytes = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = fixed_bytes;
+    fixed_bytes += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t o_perm = take(4 * n), o_clean = take(4 * n), o_start = take(16), o_cnt = take(256),
+               o_visn = take(4 * maxB), o_cmps = take(4 * maxB), o_status = take(4 * maxB),
+               o_pka = take(4 * pairs_cap), o_pkb = take(4 * pairs_cap), o_pva = take(4 * pairs_cap),
+               o_pvb = take(4 * pairs_cap), o_uniq = take(4 * pairs_cap), o_counts = take(4 * pairs_cap),
+               o_offs = take(4 * pairs_cap), o_nruns = take(16), o_jobs = take(12 * pairs_cap),
+               o_big = take(32 * big_cap), o_cub = take(cub_bytes);
+  BCUDA(bb.fixed.ensure(fixed_bytes));
+  uint8_t* const fb = bb.fixed.as<uint8_t>();
+  auto u32 = [&](size_t at) { return reinterpret_cast<uint32_t*>(fb + at); };
+  uint32_t* d_perm = u32(o_perm);
+  uint32_t *pk_a = u32(o_pka), *pk_b = u32(o_pkb), *pv_a = u32(o_pva), *pv_b = u32(o_pvb);
+  BCUDA(bb.vis_keys.ensure(8 * maxB * vis_cap));
+
+  // insertion order
+  if (perm) {
+    BCUDA(cudaMemcpyAsync(d_perm, perm, 4 * n, cudaMemcpyHostToDevice, st));
+  } else {
+    DevBuf kk;
+    BCUDA(kk.ensure(20 * n));
+    uint64_t *k1 = kk.as<uint64_t>(), *k2 = k1 + n;
+    uint32_t* i1 = reinterpret_cast<uint32_t*>(k2 + n);
+    perm_keys_kernel<<<(int)std::min<uint64_t>((n + 255) / 256, 65535), 256, 0, st>>>(k1, i1, n, bp->perm_seed);
+    size_t tb = cub_bytes;
+    const cudaError_t e = cub::DeviceRadixSort::SortPairs(fb + o_cub, tb, k1, k2, i1, d_perm, (int)n, 0, 64, st);
+    cudaStreamSynchronize(st);
+    kk.release();
+    BCUDA(e);
+  }
+
+  const uint32_t start0 = 0;
+  BCUDA(cudaMemcpyAsync(fb + o_start, &start0, 4, cudaMemcpyHostToDevice, st));
+  uint32_t* c32 = u32(o_cnt);  // [0] status or, [2] flagged count, [4..7] reverse-edge prunes per class
+  // [0] dist cmps, [1] visited, [2] class 3 segment cursor, [3] search cmps,
+  // [4] insertion prune candidates, [5] reverse-edge pairs, [6] reverse-edge prune candidates
+  unsigned long long* c64 = reinterpret_cast<unsigned long long*>(c32 + 8);
+  BCUDA(cudaMemsetAsync(fb + o_cnt, 0, 256, st));
+  BCUDA(cudaMemsetAsync(fb + o_clean, 0, 4 * n, st));
+
+  // the searches' buffers at the largest batch, so that they are not regrown batch by batch
+  pann_query_params qp{0, bp->L, n, R, bp->batch_factor};
+  SearchPlan plan;
+  {
+    int rc = make_plan(idx, &qp, 1, &plan);
+    TierSizes z;
+    TierBufs tb;
+    if (!rc) rc = size_tiers(idx, plan, maxB, PREC_F32, 0, 0, &z);
+    if (!rc) rc = index_tier_buffers(idx, z, (uint32_t)maxB, PREC_F32, &tb);
+    if (rc) { cleanup(); return rc; }
+  }
+
+  PruneArgs pa{};
+  pa.points = idx->d_points;
+  pa.stride = stride;
+  pa.nchunks = nch;
+  pa.graph = idx->d_graph;
+  pa.R = R;
+  pa.nclean = u32(o_clean);
+  pa.dist_cmps = c64;
+
+  // Jobs sorted in global memory: assemble their keys into segments, sort, prune a block per job. begin: segment
+  // starts (device); total: keys of all segments.
+  auto prune_segments = [&](uint32_t njobs, const uint32_t* jpts, const uint64_t* skeys, uint32_t sstride,
+                            const uint32_t* sids, const uint32_t* soff, const uint32_t* sn, uint32_t* begin,
+                            uint32_t* end, uint64_t total, double alpha) -> int {
+    BCUDA(bb.seg_a.ensure_grow(8 * total + 8));
+    BCUDA(bb.seg_b.ensure_grow(8 * total + 8));
+    uint64_t *sa = bb.seg_a.as<uint64_t>(), *sb = bb.seg_b.as<uint64_t>();
+    size_t need = 0;
+    cub::DeviceSegmentedSort::SortKeys(nullptr, need, sa, sb, (int)total, (int)njobs, begin, end, st);
+    BCUDA(bb.seg_tmp.ensure_grow(need + 256));
+    BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
+      constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
+      const int blocks = (int)std::min<uint32_t>((njobs + wpb - 1) / wpb, 65535);
+      assemble_kernel<DT, MT><<<blocks, 32 * wpb, wpb * stride, st>>>(idx->d_points, stride, d, nch, idx->d_graph, R,
+                                                                     njobs, jpts, skeys, sstride, sids, soff, sn, begin,
+                                                                     end, sa, c64);
+      return cudaGetLastError();
+    }));
+    BCUDA(cub::DeviceSegmentedSort::SortKeys(bb.seg_tmp.p, need, sa, sb, (int)total, (int)njobs, begin, end, st));
+    BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
+      constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
+      PruneArgs a = pa;
+      a.alpha = alpha;
+      a.pts = jpts;
+      a.njobs_host = njobs;
+      return launch_block<DT, MT, true>(idx, a, PruneSegs{begin, end, sb}, njobs, st);
+    }));
+    return PANN_OK;
+  };
+
   uint32_t batches = 0;
-  uint64_t reprunes = 0, prune_cands = 0, inserted = 0;
+  uint64_t reprunes = 0, inserted = 0;
+  double clean_alpha = 0.0;  // the alpha of the rows' clean entries
 
   for (int pass = 0; pass < bp->num_passes; pass++) {
     const double alpha = (pass == bp->num_passes - 1) ? bp->alpha : 1.0;  // index.h:173-178
+    // clean entries stay so at the same alpha; at a larger one only where distances are not negative
+    if (pass > 0 && !(alpha == clean_alpha || (metric == MT_L2 && alpha > clean_alpha)))
+      BCUDA(cudaMemsetAsync(fb + o_clean, 0, 4 * n, st));
+    clean_alpha = alpha;
+    pa.alpha = alpha;
     for (size_t b = 0; b < fl.size(); b++) {
       const uint32_t B = (uint32_t)(ce[b] - fl[b]);
       const uint32_t* pts = d_perm + fl[b];
       batches++;
       // ---- 1. search (QueryParams(0, L, n, maxDeg, rerank, batch_factor), index.h:251-252)
-      pann_query_params qp{0, bp->L, n, R, bp->batch_factor};
-      SearchPlan plan;
-      {
-        int rc = make_plan(idx, &qp, 1, &plan);
-        if (rc) { cleanup(); return rc; }
-      }
       uint32_t sor = 0;
       for (;;) {
         BCUDA(cudaEventRecord(ea, st));
         BCUDA(cudaMemsetAsync(c32, 0, 4, st));
-        int rc = run_search(idx, plan, nullptr, pts, B, bb.start.as<uint32_t>(), nullptr, nullptr,
-                            bb.vis_n.as<uint32_t>(), bb.cmps.as<uint32_t>(), bb.status.as<uint32_t>(),
-                            bb.vis_keys.as<uint64_t>(), vis_cap, st);
+        int rc = run_search(idx, plan, nullptr, pts, B, u32(o_start), nullptr, nullptr, u32(o_visn), u32(o_cmps),
+                            u32(o_status), bb.vis_keys.as<uint64_t>(), vis_cap, st);
         if (rc) { cleanup(); return rc; }
-        status_or_kernel<<<64, 256, 0, st>>>(bb.status.as<uint32_t>(), B, c32);
+        status_or_kernel<<<64, 256, 0, st>>>(u32(o_status), B, c32);
         BCUDA(cudaMemcpyAsync(&sor, c32, 4, cudaMemcpyDeviceToHost, st));
         BCUDA(cudaEventRecord(eb, st));
         BCUDA(cudaStreamSynchronize(st));
@@ -692,8 +612,7 @@ extern "C" int pann_build(pann_index* idx, const pann_build_params* bp, const ui
         }
         if (sor & QS_VISIT_OVERFLOW) {
           vis_cap *= 2;
-          int rc2 = alloc_batch(vis_cap);
-          if (rc2) return rc2;
+          BCUDA(bb.vis_keys.ensure(8 * maxB * vis_cap));
           continue;
         }
         break;
@@ -703,113 +622,133 @@ extern "C" int pann_build(pann_index* idx, const pann_build_params* bp, const ui
         cudaEventElapsedTime(&ms, ea, eb);
         t_search += ms * 1e-3;
       }
-      count_flag_kernel<<<64, 256, 0, st>>>(bb.status.as<uint32_t>(), B, QS_REF_WOULD_GROW, c32 + 2);
-      sum_kernel<<<64, 256, 0, st>>>(bb.cmps.as<uint32_t>(), B, c64);
-      sum_kernel<<<64, 256, 0, st>>>(bb.cmps.as<uint32_t>(), B, c64 + 3);
-      sum_kernel<<<64, 256, 0, st>>>(bb.vis_n.as<uint32_t>(), B, c64 + 1);
-      // ---- 2. robustPrune of the inserted points
       BCUDA(cudaEventRecord(ea, st));
+      batch_sums_kernel<<<64, 256, 0, st>>>(u32(o_status), QS_REF_WOULD_GROW, u32(o_cmps), u32(o_visn), B, c32 + 2, c64);
+      // ---- 2. robustPrune of the inserted points
       const uint32_t segcap = vis_cap + R;
-      iota_begin_kernel<<<(B + 255) / 256, 256, 0, st>>>(bb.seg_begin.as<uint32_t>(), B, segcap);
-      BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
-        constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
-        int blocks = (int)std::min<uint32_t>((B + wpb - 1) / wpb, 65535);
-        assemble_kernel<DT, MT><<<blocks, 32 * wpb, wpb * warp_smem, st>>>(
-            idx->d_points, stride, d, nch, idx->d_graph, R, B, pts, bb.vis_keys.as<uint64_t>(), vis_cap, nullptr,
-            nullptr, bb.vis_n.as<uint32_t>(), bb.seg_begin.as<uint32_t>(), bb.seg_end.as<uint32_t>(),
-            bb.seg_a.as<uint64_t>(), c64);
-        return cudaGetLastError();
-      }));
-      {
-        size_t tb = bb.cub_tmp.bytes;
-        BCUDA(cub::DeviceSegmentedSort::SortKeys(bb.cub_tmp.p, tb, bb.seg_a.as<uint64_t>(), bb.seg_b.as<uint64_t>(),
-                                                 (int)((uint64_t)B * segcap), (int)B, bb.seg_begin.as<uint32_t>(),
-                                                 bb.seg_end.as<uint32_t>(), st));
+      if (!blocks_only && prune_wpb(idx, prune_warp_bytes(stride, segcap, scratch)) > 0) {
+        BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
+          constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
+          PruneArgs a = pa;
+          a.pts = pts;
+          a.njobs_host = B;
+          a.src_keys = bb.vis_keys.as<uint64_t>();
+          a.src_keys_stride = vis_cap;
+          a.src_n = u32(o_visn);
+          a.cap = segcap;
+          a.cands = c64 + 4;
+          return launch_lazy<DT, MT>(idx, a, B, st);
+        }));
+      } else {
+        // candidate lists too long for a warp's shared memory
+        BCUDA(bb.seg_se.ensure(8 * maxB));
+        uint32_t *sbeg = bb.seg_se.as<uint32_t>(), *send = sbeg + maxB;
+        iota_begin_kernel<<<(B + 255) / 256, 256, 0, st>>>(sbeg, B, segcap);
+        int rc = prune_segments(B, pts, bb.vis_keys.as<uint64_t>(), vis_cap, nullptr, nullptr, u32(o_visn), sbeg, send,
+                                (uint64_t)B * segcap, alpha);
+        if (rc) return rc;
+        seg_len_sum_kernel<<<64, 256, 0, st>>>(sbeg, send, B, c64 + 4);
       }
-      BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
-        constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
-        return launch_greedy<DT, MT>(idx, B, pts, bb.seg_begin.as<uint32_t>(), bb.seg_end.as<uint32_t>(),
-                                     bb.seg_b.as<uint64_t>(), alpha, c64, false, st);
-      }));
       BCUDA(cudaEventRecord(eb, st));
-      seg_len_sum_kernel<<<64, 256, 0, st>>>(bb.seg_begin.as<uint32_t>(), bb.seg_end.as<uint32_t>(), B, c64 + 4);
       degree_sum_kernel<<<128, 256, 0, st>>>(idx->d_graph, R, pts, B, c64 + 5);
       // ---- 3. reverse edges
       const uint64_t np = (uint64_t)B * R;
-      reverse_pairs_kernel<<<(int)std::min<uint64_t>((np + 255) / 256, 65535), 256, 0, st>>>(
-          idx->d_graph, R, pts, B, bb.pk_a.as<uint32_t>(), bb.pv_a.as<uint32_t>());
+      reverse_pairs_kernel<<<(int)std::min<uint64_t>((np + 255) / 256, 65535), 256, 0, st>>>(idx->d_graph, R, pts, B,
+                                                                                             (uint32_t)n, pk_a, pv_a);
       {
-        size_t tb = bb.cub_tmp.bytes;
-        int bits = 1;
-        while (bits < 32 && (1ull << bits) <= n) bits++;
-        // PAD (all ones) must still sort last: sort all 32 bits when n needs fewer
-        BCUDA(cub::DeviceRadixSort::SortPairs(bb.cub_tmp.p, tb, bb.pk_a.as<uint32_t>(), bb.pk_b.as<uint32_t>(),
-                                              bb.pv_a.as<uint32_t>(), bb.pv_b.as<uint32_t>(), (int)np, 0, 32, st));
-        tb = bb.cub_tmp.bytes;
-        BCUDA(cub::DeviceRunLengthEncode::Encode(bb.cub_tmp.p, tb, bb.pk_b.as<uint32_t>(), bb.uniq.as<uint32_t>(),
-                                                 bb.counts.as<uint32_t>(), bb.nruns.as<uint32_t>(), (int)np, st));
-        tb = bb.cub_tmp.bytes;
-        BCUDA(cub::DeviceScan::ExclusiveSum(bb.cub_tmp.p, tb, bb.counts.as<uint32_t>(), bb.offs.as<uint32_t>(),
-                                            (int)np, st));
+        size_t tb = cub_bytes;
+        BCUDA(cub::DeviceRadixSort::SortPairs(fb + o_cub, tb, pk_a, pk_b, pv_a, pv_b, (int)np, 0, key_bits, st));
+        tb = cub_bytes;
+        BCUDA(cub::DeviceRunLengthEncode::Encode(fb + o_cub, tb, pk_b, u32(o_uniq), u32(o_counts), u32(o_nruns), (int)np,
+                                                 st));
+        tb = cub_bytes;
+        BCUDA(cub::DeviceScan::ExclusiveSum(fb + o_cub, tb, u32(o_counts), u32(o_offs), (int)np, st));
       }
-      BCUDA(cudaMemsetAsync(c32 + 1, 0, 4, st));
+      BCUDA(cudaMemsetAsync(c32 + 4, 0, 16, st));
       BCUDA(cudaMemsetAsync(c64 + 2, 0, 8, st));
-      {
-        int blocks = (int)std::min<uint64_t>((np * 32 + 255) / 256, 65535);
-        reverse_classify_kernel<<<blocks, 256, 0, st>>>(idx->d_graph, R, bb.uniq.as<uint32_t>(),
-                                                        bb.counts.as<uint32_t>(), bb.offs.as<uint32_t>(),
-                                                        bb.nruns.as<uint32_t>(), bb.pv_b.as<uint32_t>(),
-                                                        bb.jobs.as<uint32_t>(), bb.job_off.as<uint32_t>(),
-                                                        bb.job_n.as<uint32_t>(), bb.seg_begin.as<uint32_t>(), c32 + 1,
-                                                        c64 + 2);
-        BCUDA(cudaGetLastError());
-      }
-      uint32_t njobs = 0;
+      ClassifyArgs ca{};
+      ca.graph = idx->d_graph;
+      ca.R = R;
+      ca.n = (uint32_t)n;
+      ca.nclean = pa.nclean;
+      ca.uniq = u32(o_uniq);
+      ca.counts = u32(o_counts);
+      ca.offs = u32(o_offs);
+      ca.num_runs = u32(o_nruns);
+      ca.vals = pv_b;
+      ca.job_pts = u32(o_jobs);
+      ca.job_off = ca.job_pts + pairs_cap;
+      ca.job_n = ca.job_off + pairs_cap;
+      ca.jobs_cap = (uint32_t)pairs_cap;
+      ca.big_pts = u32(o_big);
+      ca.big_off = ca.big_pts + 2 * big_cap;
+      ca.big_n = ca.big_off + 2 * big_cap;
+      ca.big_begin = ca.big_n + 2 * big_cap;
+      ca.big_cap = (uint32_t)big_cap;
+      ca.njobs = c32 + 4;
+      ca.seg_total = c64 + 2;
+      ca.cands_total = c64 + 6;
+      ca.cap0 = reprune_ok ? cap0 : 0;
+      ca.dcap = dcap;
+      ca.cap1 = cap1;
+      ca.cap2 = cap2;
+      reverse_classify_kernel<<<(int)std::min<uint64_t>((np * 32 + 255) / 256, 65535), 256, 0, st>>>(ca);
+      BCUDA(cudaGetLastError());
+      const uint64_t max_jobs = std::min<uint64_t>(np, n);
+      BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
+        constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
+        PruneArgs a = pa;
+        a.src_ids = pv_b;
+        a.pts = ca.job_pts;
+        a.src_off = ca.job_off;
+        a.src_n = ca.job_n;
+        cudaError_t e = cudaSuccess;
+        // the long jobs first
+        if ((uint64_t)B + R > cap1) {
+          PruneArgs c = a;
+          c.pts = ca.big_pts;
+          c.src_off = ca.big_off;
+          c.src_n = ca.big_n;
+          c.njobs = c32 + 6;
+          c.cap = cap2;
+          e = launch_block<DT, MT, false>(idx, c, PruneSegs{}, lazy_ok ? max_jobs / 64 + 1 : max_jobs, st);
+          if (e != cudaSuccess) return e;
+        }
+        if (lazy_ok) {
+          PruneArgs c = a;
+          c.njobs = c32 + 5;
+          c.flip = (uint32_t)pairs_cap - 1;
+          c.cap = cap1;
+          e = launch_lazy<DT, MT>(idx, c, max_jobs, st);
+          if (e != cudaSuccess) return e;
+        }
+        if (reprune_ok) {
+          a.njobs = c32 + 4;
+          a.cap = cap0;
+          a.dcap = dcap;
+          e = launch_reprune<DT, MT>(idx, a, max_jobs, st);
+        }
+        return e;
+      }));
+      uint32_t nj[4] = {0, 0, 0, 0};
       unsigned long long seg_total = 0;
-      BCUDA(cudaMemcpyAsync(&njobs, c32 + 1, 4, cudaMemcpyDeviceToHost, st));
+      BCUDA(cudaMemcpyAsync(nj, c32 + 4, 16, cudaMemcpyDeviceToHost, st));
       BCUDA(cudaMemcpyAsync(&seg_total, c64 + 2, 8, cudaMemcpyDeviceToHost, st));
-      BCUDA(cudaStreamSynchronize(st));
-      reprunes += njobs;
-      prune_cands += seg_total;
-      inserted += B;
-      if (njobs) {
+      BCUDA(cudaEventRecord(ec, st));
+      BCUDA(cudaEventSynchronize(ec));
+      if (nj[3]) {
         if (seg_total >= 0x7FFFFFFFull) {
           cleanup();
           return fail(PANN_ENOMEM, "reverse-edge prune segments exceed 2^31 keys");
         }
-        // scratch for exactly seg_total keys (grown if this batch needs more)
-        BCUDA(bb.seg_a.ensure_grow(8 * seg_total + 8));
-        BCUDA(bb.seg_b.ensure_grow(8 * seg_total + 8));
-        {
-          size_t need = 0;
-          cub::DeviceSegmentedSort::SortKeys(nullptr, need, bb.seg_a.as<uint64_t>(), bb.seg_b.as<uint64_t>(),
-                                             (int)seg_total, (int)njobs, bb.seg_begin.as<uint32_t>(),
-                                             bb.seg_end.as<uint32_t>(), st);
-          BCUDA(bb.cub_tmp.ensure_grow(need + 256));
-        }
-        BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
-          constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
-          int blocks = (int)std::min<uint32_t>((njobs + wpb - 1) / wpb, 65535);
-          assemble_kernel<DT, MT><<<blocks, 32 * wpb, wpb * warp_smem, st>>>(
-              idx->d_points, stride, d, nch, idx->d_graph, R, njobs, bb.jobs.as<uint32_t>(), nullptr, 0,
-              bb.pv_b.as<uint32_t>(), bb.job_off.as<uint32_t>(), bb.job_n.as<uint32_t>(), bb.seg_begin.as<uint32_t>(),
-              bb.seg_end.as<uint32_t>(), bb.seg_a.as<uint64_t>(), c64);
-          return cudaGetLastError();
-        }));
-        {
-          size_t tb = bb.cub_tmp.bytes;
-          BCUDA(cub::DeviceSegmentedSort::SortKeys(bb.cub_tmp.p, tb, bb.seg_a.as<uint64_t>(), bb.seg_b.as<uint64_t>(),
-                                                   (int)seg_total, (int)njobs, bb.seg_begin.as<uint32_t>(),
-                                                   bb.seg_end.as<uint32_t>(), st));
-        }
-        BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
-          constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
-          return launch_greedy<DT, MT>(idx, njobs, bb.jobs.as<uint32_t>(), bb.seg_begin.as<uint32_t>(),
-                                       bb.seg_end.as<uint32_t>(), bb.seg_b.as<uint64_t>(), alpha, c64, true, st);
-        }));
+        int rc = prune_segments(nj[3], ca.big_pts + big_cap, nullptr, 0, pv_b, ca.big_off + big_cap, ca.big_n + big_cap,
+                                ca.big_begin, ca.big_begin + big_cap, seg_total, alpha);
+        if (rc) return rc;
+        BCUDA(cudaEventRecord(ec, st));
+        BCUDA(cudaEventSynchronize(ec));
       }
-      BCUDA(cudaEventRecord(ec, st));
-      BCUDA(cudaEventSynchronize(ec));
+      reprunes += (uint64_t)nj[0] + nj[1] + nj[2] + nj[3];
+      inserted += B;
       {
         float ms = 0;
         cudaEventElapsedTime(&ms, ea, eb);
@@ -822,7 +761,7 @@ extern "C" int pann_build(pann_index* idx, const pann_build_params* bp, const ui
   if (bp->sort_neighbors) {
     BCUDA(dispatch_dm(dtype, metric, [&](auto DTc, auto MTc) {
       constexpr int DT = decltype(DTc)::value, MT = decltype(MTc)::value;
-      size_t sm = wpb * (stride + 16ull * R);
+      size_t sm = wpb * (stride + scratch + 16ull * R);
       auto kern = sort_neighbors_kernel<DT, MT>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
       int blocks = (int)std::min<uint64_t>((n + wpb - 1) / wpb, 65535ull * 8);
@@ -840,16 +779,16 @@ extern "C" int pann_build(pann_index* idx, const pann_build_params* bp, const ui
     stats->search_seconds = t_search;
     stats->prune_seconds = t_prune;
     stats->reverse_seconds = t_rev;
-    unsigned long long h64[6] = {0, 0, 0, 0, 0, 0};
+    unsigned long long h64[7] = {0, 0, 0, 0, 0, 0, 0};
     uint32_t h32[4] = {0, 0, 0, 0};
-    cudaMemcpy(h64, c64, 48, cudaMemcpyDeviceToHost);
+    cudaMemcpy(h64, c64, 56, cudaMemcpyDeviceToHost);
     cudaMemcpy(h32, c32, 16, cudaMemcpyDeviceToHost);
     stats->dist_cmps = h64[0];
     stats->visited_total = h64[1];
     stats->batches = batches;
     stats->flagged = h32[2];
     stats->search_cmps = h64[3];
-    stats->prune_candidates = h64[4] + prune_cands;
+    stats->prune_candidates = h64[4] + h64[6];
     stats->edge_pairs = h64[5];
     stats->reprunes = reprunes;
     stats->inserted = inserted;
