@@ -174,8 +174,8 @@ static uint32_t pow2_at_least(uint64_t x) {
   return p;
 }
 
-// Tier-0 register budget for float32 Euclidean search: PANN_T0_MINB=4 fits the
-// kernel to four 128-thread blocks per SM (128 registers) instead of three.
+// Tier-0 register budget: PANN_T0_MINB=4 fits the kernel to six 128-thread
+// blocks per SM (80 registers) instead of four (128).
 static int t0_minb() {
   static const int v = [] {
     const char* e = std::getenv("PANN_T0_MINB");
@@ -184,32 +184,32 @@ static int t0_minb() {
   return v;
 }
 
-// The first tier's kernel fitted to `minb` resident 128-thread blocks (3 or 4).
-template <int DT, int MT, bool G, int PREC = PREC_F32>
+// The first tier's kernel for a register budget: `minb` 3 (four resident 128-thread blocks) or 4 (six).
+template <int DT, int MT, int SEEN, int PREC = PREC_F32>
 static auto search_kernel_ptr(int minb) {
-  if constexpr (!G && PREC == PREC_F32)
-    if (minb == 4) return search_kernel<DT, MT, G, PREC, 4>;
-  return search_kernel<DT, MT, G, PREC, 3>;
+  if constexpr (SEEN != SEEN_GLOBAL && PREC == PREC_F32)
+    if (minb == 4) return search_kernel<DT, MT, SEEN, PREC, 6>;
+  return search_kernel<DT, MT, SEEN, PREC, PREC == PREC_F32 ? 4 : 3>;
 }
 
-template <int DT, int MT, bool G, int PREC = PREC_F32>
+template <int DT, int MT, int SEEN, int PREC = PREC_F32>
 static cudaError_t launch_search_t(const SearchArgs& a, int blocks, int threads, size_t smem, cudaStream_t st,
                                    int minb) {
-  auto k = search_kernel_ptr<DT, MT, G, PREC>(minb);
+  auto k = search_kernel_ptr<DT, MT, SEEN, PREC>(minb);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
   if (e != cudaSuccess) return e;
   k<<<blocks, threads, smem, st>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_search(int dtype, int metric, bool global_table, const SearchArgs& a, int blocks,
+cudaError_t launch_search(int dtype, int metric, int seen, const SearchArgs& a, int blocks,
                                  int threads, size_t smem, cudaStream_t st, int prec, int minb) {
   if (prec != PREC_F32) {
     if (dtype != DT_F32) return cudaErrorInvalidValue;
 #define PANN_LP_CASE(MT, PR)                                                               \
     if (metric == MT && prec == PR)                                                        \
-      return global_table ? launch_search_t<DT_F32, MT, true, PR>(a, blocks, threads, smem, st, 3) \
-                          : launch_search_t<DT_F32, MT, false, PR>(a, blocks, threads, smem, st, 3);
+      return seen == SEEN_GLOBAL ? launch_search_t<DT_F32, MT, SEEN_GLOBAL, PR>(a, blocks, threads, smem, st, 3) \
+                                 : launch_search_t<DT_F32, MT, SEEN32, PR>(a, blocks, threads, smem, st, 3);
     PANN_LP_CASE(MT_L2, PREC_BF16)
     PANN_LP_CASE(MT_IP, PREC_BF16)
     PANN_LP_CASE(MT_L2, PREC_FP8)
@@ -219,8 +219,9 @@ cudaError_t launch_search(int dtype, int metric, bool global_table, const Search
   }
 #define PANN_SEARCH_CASE(DT, MT)                                                        \
   if (dtype == DT && metric == MT)                                                      \
-    return global_table ? launch_search_t<DT, MT, true>(a, blocks, threads, smem, st, 3)   \
-                        : launch_search_t<DT, MT, false>(a, blocks, threads, smem, st, minb);
+    return seen == SEEN_GLOBAL ? launch_search_t<DT, MT, SEEN_GLOBAL>(a, blocks, threads, smem, st, 3) \
+           : seen == SEEN16    ? launch_search_t<DT, MT, SEEN16>(a, blocks, threads, smem, st, minb)   \
+                               : launch_search_t<DT, MT, SEEN32>(a, blocks, threads, smem, st, minb);
   PANN_SEARCH_CASE(DT_U8, MT_L2)
   PANN_SEARCH_CASE(DT_U8, MT_IP)
   PANN_SEARCH_CASE(DT_I8, MT_L2)
@@ -278,18 +279,19 @@ cudaError_t launch_emulate_block(int dtype, int metric, const SearchArgs& a, con
   return cudaErrorInvalidValue;
 }
 
-template <int DT, int MT, bool G, int PREC = PREC_F32>
+template <int DT, int MT, int SEEN, int PREC = PREC_F32>
 static int occupancy_t(int threads, size_t smem, int minb = 3) {
   int nb = 0;
-  auto k = search_kernel_ptr<DT, MT, G, PREC>(minb);
+  auto k = search_kernel_ptr<DT, MT, SEEN, PREC>(minb);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem) != cudaSuccess) return 0;
   return nb;
 }
-int search_occupancy(int dtype, int metric, bool g, int threads, size_t smem, int minb) {
-#define PANN_OCC_CASE(DT, MT) \
-  if (dtype == DT && metric == MT) \
-    return g ? occupancy_t<DT, MT, true>(threads, smem) : occupancy_t<DT, MT, false>(threads, smem, minb);
+static int search_occupancy(int dtype, int metric, int seen, int threads, size_t smem, int minb) {
+#define PANN_OCC_CASE(DT, MT)                                                                     \
+  if (dtype == DT && metric == MT)                                                                \
+    return seen == SEEN16 ? occupancy_t<DT, MT, SEEN16>(threads, smem, minb)                      \
+                          : occupancy_t<DT, MT, SEEN32>(threads, smem, minb);
   PANN_OCC_CASE(DT_U8, MT_L2)
   PANN_OCC_CASE(DT_U8, MT_IP)
   PANN_OCC_CASE(DT_I8, MT_L2)
@@ -301,10 +303,10 @@ int search_occupancy(int dtype, int metric, bool g, int threads, size_t smem, in
 }
 
 static int lp_occupancy(int metric, int prec, int threads, size_t smem) {
-  if (metric == MT_L2 && prec == PREC_BF16) return occupancy_t<DT_F32, MT_L2, false, PREC_BF16>(threads, smem);
-  if (metric == MT_IP && prec == PREC_BF16) return occupancy_t<DT_F32, MT_IP, false, PREC_BF16>(threads, smem);
-  if (metric == MT_L2 && prec == PREC_FP8) return occupancy_t<DT_F32, MT_L2, false, PREC_FP8>(threads, smem);
-  if (metric == MT_IP && prec == PREC_FP8) return occupancy_t<DT_F32, MT_IP, false, PREC_FP8>(threads, smem);
+  if (metric == MT_L2 && prec == PREC_BF16) return occupancy_t<DT_F32, MT_L2, SEEN32, PREC_BF16>(threads, smem);
+  if (metric == MT_IP && prec == PREC_BF16) return occupancy_t<DT_F32, MT_IP, SEEN32, PREC_BF16>(threads, smem);
+  if (metric == MT_L2 && prec == PREC_FP8) return occupancy_t<DT_F32, MT_L2, SEEN32, PREC_FP8>(threads, smem);
+  if (metric == MT_IP && prec == PREC_FP8) return occupancy_t<DT_F32, MT_IP, SEEN32, PREC_FP8>(threads, smem);
   return 0;
 }
 
@@ -327,6 +329,71 @@ uint32_t tier0_slots(const SearchPlan& p, uint32_t R) {
   return std::max<uint32_t>(s, floor_s);
 }
 
+// Tier 0's shape. The seen table takes 16 bits an entry where the index's ids
+// fit (SEEN16_REM bits past the slot number: 8M points at 4,096 slots), 32
+// otherwise. Warps a block: few queries are spread over the SMs first (a warp
+// alone on an SM has its L1 and issue slots to itself); many take the count
+// that leaves the most warps resident.
+int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
+                int wpb_force, int minb, TierSizes* z) {
+  const size_t cap = idx->smem_optin;
+  const uint32_t S_min = pow2_at_least(4ull * (idx->R + 1));
+  uint32_t S = S_force ? std::max<uint32_t>(pow2_at_least(S_force), S_min) : tier0_slots(plan, idx->R);
+  z->scratch = precision == PREC_F32 ? row_score_scratch_rt(idx->dtype) : 0u;
+  uint32_t nbits = 1;
+  while (nbits < 31 && (1ull << nbits) < idx->n) nbits++;
+  // with at most 12 queries an SM the wider table fits anyway, and probing it takes fewer instructions
+  const bool many = S_force != 0 || wpb_force != 0 || nq > 12ull * idx->sm_count;
+  auto shape = [&]() {
+    uint32_t sbits = 0;
+    while ((1u << sbits) < S) sbits++;
+    z->seen = precision == PREC_F32 && many && nbits <= sbits + SEEN16_REM ? SEEN16 : SEEN32;
+    z->id_bits = std::max(nbits, sbits);
+    z->wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, z->seen, z->scratch);
+  };
+  shape();
+  while (z->wb > cap && S > S_min) {
+    S >>= 1;
+    shape();
+  }
+  if (z->wb > cap) return fail(PANN_EINVAL, "search state for this beam does not fit in shared memory");
+  // few queries: a table less full takes fewer probes
+  if (!many && S_force == 0 && !std::getenv("PANN_SEEN_SLOTS")) {
+    const size_t room = (200ull << 10) / std::max<uint64_t>(1, (nq + idx->sm_count - 1) / idx->sm_count);
+    for (int g = 0; g < 2 && S < 8192 && z->wb + 4ull * S <= std::min(room, cap); g++) {
+      S <<= 1;
+      shape();
+    }
+  }
+  auto occ_of = [&](int w) {
+    if ((size_t)z->wb * w > cap) return 0;
+    const int o = precision == PREC_F32
+                      ? search_occupancy(idx->dtype, idx->metric, z->seen, 32 * w, (size_t)z->wb * w, minb)
+                      : lp_occupancy(idx->metric, precision, 32 * w, (size_t)z->wb * w);
+    return std::max(o, 1);
+  };
+  int wpb = 0, occ = 0;
+  if (wpb_force > 0) {
+    wpb = std::min(wpb_force, 4);
+    while (wpb > 1 && (size_t)z->wb * wpb > cap) wpb >>= 1;
+    occ = occ_of(wpb);
+  } else {
+    const int most = (int)std::min<uint64_t>(4, (std::max<uint64_t>(nq, 1) + idx->sm_count - 1) / idx->sm_count);
+    for (int w = most; w >= 1; w--) {
+      const int o = occ_of(w);
+      if (o * w > occ * wpb) {
+        wpb = w;
+        occ = o;
+      }
+    }
+  }
+  z->S = S;
+  z->wpb = wpb;
+  z->blocks = (int)std::min<uint64_t>((std::max<uint64_t>(nq, 1) + wpb - 1) / wpb, (uint64_t)occ * idx->sm_count);
+  z->slots = (size_t)z->blocks * wpb;
+  return PANN_OK;
+}
+
 // Tiers: (0) every query, many warps per SM, shared-memory seen table with a
 // global spill table; (2) queries whose tables still filled up, with one large
 // global table per warp; (E) queries on which the reference's hashset grows,
@@ -337,26 +404,10 @@ int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int p
   TierSizes& t = *z;
   t = TierSizes{};
   // ---- tier 0
-  uint32_t S = S_force ? std::max<uint32_t>(pow2_at_least(S_force), pow2_at_least(4ull * (idx->R + 1)))
-                       : tier0_slots(plan, idx->R);
-  uint32_t wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, false);
-  int wpb = wpb_force > 0 ? std::min(wpb_force, 4) : 4;
-  while (wpb > 1 && (size_t)wb * wpb > smem_cap) wpb >>= 1;
-  while ((size_t)wb * wpb > smem_cap && S > pow2_at_least(4ull * (idx->R + 1))) {
-    S >>= 1;
-    wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, false);
-  }
-  if ((size_t)wb * wpb > smem_cap) return fail(PANN_EINVAL, "search state for this beam does not fit in shared memory");
   t.minb = precision == PREC_F32 ? (minb_force == 4 || (minb_force == 0 && t0_minb() == 4) ? 4 : 3) : 3;
-  int occ = precision == PREC_F32 ? search_occupancy(idx->dtype, idx->metric, false, 32 * wpb, (size_t)wb * wpb, t.minb)
-                                  : lp_occupancy(idx->metric, precision, 32 * wpb, (size_t)wb * wpb);
-  if (occ <= 0) occ = 1;
-  uint64_t want = (std::max<uint64_t>(nq, 1) + wpb - 1) / wpb;
-  t.S = S;
-  t.wb = wb;
-  t.wpb = wpb;
-  t.blocks = (int)std::min<uint64_t>(want, (uint64_t)occ * idx->sm_count);
-  t.slots = (size_t)t.blocks * wpb;
+  int rc0 = tier0_shape(idx, plan, nq, precision, S_force, wpb_force, t.minb, &t);
+  if (rc0) return rc0;
+  const uint32_t S = t.S;
   uint32_t Sg = std::max<uint32_t>(4 * S, pow2_at_least(2ull * plan.ref_half));
   while (Sg > 4 * S && t.slots * Sg * 4 > (1ull << 30)) Sg >>= 1;
   t.Sg = Sg;
@@ -370,14 +421,14 @@ int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int p
   // ---- tier 2
   t.S2 = std::min<uint32_t>(std::max<uint32_t>(1u << 16, pow2_at_least(4ull * plan.ref_half)), 1u << 24);
   t.t2_slots = (int)std::max<uint64_t>(1, std::min<uint64_t>(2ull * idx->sm_count, (256ull << 20) / (4ull * t.S2)));
-  t.wb2 = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, t.S2, true);
+  t.wb2 = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, t.S2, SEEN_GLOBAL, t.scratch);
   t.t2_bytes = (size_t)t.t2_slots * t.S2 * 4;
   // ---- emulation tiers
   double cap_n = 2.0 * (10.0 + (double)plan.L) * (double)plan.dl;
   t.bits0 = (uint32_t)std::ceil(std::log2(cap_n));
   t.S0 = 1ull << t.bits0;
   t.vs = pow2_at_least(8ull * plan.L + 64);
-  t.base = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, 0, true);
+  t.base = emu_state_bytes(idx->stride, plan.L, plan.Ccap, idx->R);
   t.emu_smem_need = emu_block_layout(idx->stride, plan.L, plan.Ccap, idx->R, t.vs, (uint32_t)(4 * t.S0),
                                      (uint32_t)(2 * t.S0)).bytes;
   t.emu_smem = 4 * t.S0 < (1ull << 30) && t.emu_smem_need <= smem_cap;
@@ -402,6 +453,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
     PANN_CUDA(cudaStreamWaitEvent(side, idx->ev_fork, 0));
   }
   SearchArgs a = a0;
+  a.scr_bytes = search_scr_bytes(a.L, a.Ccap, z.scratch);
   a.emu_list = b.emu;
   a.emu_rec = b.emu_rec;
   a.emu_count = cnt + 6;
@@ -419,6 +471,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
   {
     SearchArgs t = a;
     t.S = z.S;
+    t.id_bits = z.id_bits;
     t.warp_bytes = z.wb;
     t.job_counter = cnt + 0;
     t.job_list = b.job_list0;
@@ -483,7 +536,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
                                emu_smem_bytes(z.base, z.vs, 0, 0, false), st));
       return PANN_OK;
     }
-    PANN_CUDA(launch_search(idx->dtype, idx->metric, false, t, z.blocks, 32 * z.wpb, (size_t)z.wb * z.wpb, st, precision,
+    PANN_CUDA(launch_search(idx->dtype, idx->metric, z.seen, t, z.blocks, 32 * z.wpb, (size_t)z.wb * z.wpb, st, precision,
                             z.minb));
   }
   if (early) {
@@ -523,7 +576,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
     t.job_counter = cnt + 2;
     t.redo_list = nullptr;
     t.redo_count = nullptr;
-    PANN_CUDA(launch_search(idx->dtype, idx->metric, true, t, z.t2_slots, 32, z.wb2, st, precision));
+    PANN_CUDA(launch_search(idx->dtype, idx->metric, SEEN_GLOBAL, t, z.t2_slots, 32, z.wb2, st, precision));
   }
   if (precision != PREC_F32) return PANN_OK;
   // ---- tier E: exact emulation of the reference's hashset for flagged queries,

@@ -128,30 +128,10 @@ __device__ __forceinline__ float dist_int_row(const uint4* __restrict__ row, con
 // float32 terms. For Euclidean distance the staged query holds -q, so the
 // difference is formed as x + (-q) = x - q (exact negation, same rounding as
 // q - x) and (x - q)^2 == (q - x)^2 bit for bit; for mips the query holds q.
-template <int MT>
-__device__ __forceinline__ float f32_chunk(float r, float4 a, float4 qc) {
-  if (MT == MT_L2) {
-    float t;
-    t = __fadd_rn(a.x, qc.x); r = __fadd_rn(r, __fmul_rn(t, t));
-    t = __fadd_rn(a.y, qc.y); r = __fadd_rn(r, __fmul_rn(t, t));
-    t = __fadd_rn(a.z, qc.z); r = __fadd_rn(r, __fmul_rn(t, t));
-    t = __fadd_rn(a.w, qc.w); r = __fadd_rn(r, __fmul_rn(t, t));
-  } else {
-    r = __fadd_rn(r, __fmul_rn(qc.x, a.x));
-    r = __fadd_rn(r, __fmul_rn(qc.y, a.y));
-    r = __fadd_rn(r, __fmul_rn(qc.z, a.z));
-    r = __fadd_rn(r, __fmul_rn(qc.w, a.w));
-  }
-  return r;
-}
-
-// Two rows in one packed f32x2 chain (sm_100 paired FP32): add.rn.f32x2 and
-// mul.rn.f32x2 round every component to nearest like the scalar operations.
-// The backend nevertheless fuses a paired multiply feeding a paired add into
-// one fused multiply-add (measured on sm_100a), which rounds the product
-// away. Each product is therefore OR-ed with `opq`, a zero the compiler cannot
-// see (it arrives as a kernel argument), so the add's operand is no longer a
-// multiply result and the two roundings of the reference stay separate.
+// Differences and products of neighbouring dimensions go two at a time (sm_100
+// paired FP32: both components rounded to nearest like the scalar operations),
+// the sum stays one scalar chain: 8 instructions a chunk instead of 12, and a
+// row's score is what the search kernels spend most instructions on.
 __device__ __forceinline__ uint64_t pk2(float lo, float hi) {
   return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
 }
@@ -165,6 +145,30 @@ __device__ __forceinline__ uint64_t mul2_rn(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+template <int MT>
+__device__ __forceinline__ float f32_chunk(float r, float4 a, float4 qc) {
+  uint64_t p0, p1;
+  if (MT == MT_L2) {
+    const uint64_t t0 = add2_rn(pk2(a.x, a.y), pk2(qc.x, qc.y)), t1 = add2_rn(pk2(a.z, a.w), pk2(qc.z, qc.w));
+    p0 = mul2_rn(t0, t0);
+    p1 = mul2_rn(t1, t1);
+  } else {
+    p0 = mul2_rn(pk2(qc.x, qc.y), pk2(a.x, a.y));
+    p1 = mul2_rn(pk2(qc.z, qc.w), pk2(a.z, a.w));
+  }
+  r = __fadd_rn(r, __uint_as_float((uint32_t)p0));
+  r = __fadd_rn(r, __uint_as_float((uint32_t)(p0 >> 32)));
+  r = __fadd_rn(r, __uint_as_float((uint32_t)p1));
+  return __fadd_rn(r, __uint_as_float((uint32_t)(p1 >> 32)));
+}
+
+// Two rows in one packed f32x2 chain (sm_100 paired FP32): add.rn.f32x2 and
+// mul.rn.f32x2 round every component to nearest like the scalar operations.
+// The backend nevertheless fuses a paired multiply feeding a paired add into
+// one fused multiply-add (measured on sm_100a), which rounds the product
+// away. Each product is therefore OR-ed with `opq`, a zero the compiler cannot
+// see (it arrives as a kernel argument), so the add's operand is no longer a
+// multiply result and the two roundings of the reference stay separate.
 template <int MT>
 __device__ __forceinline__ uint64_t f32_chunk2(uint64_t r, float4 a, float4 b, float4 qc, uint64_t opq) {
   if (MT == MT_L2) {

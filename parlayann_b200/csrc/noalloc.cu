@@ -32,16 +32,9 @@
 #include "index.cuh"
 #include "search.cuh"
 #include "search_emu.cuh"
+#include "tiers.cuh"
 
 namespace pann {
-
-// defined in capi.cu
-cudaError_t launch_search(int dtype, int metric, bool global_table, const SearchArgs& a, int blocks, int threads,
-                          size_t smem, cudaStream_t st, int prec, int minb = 3);
-cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
-                           int blocks, size_t smem, cudaStream_t st);
-int search_occupancy(int dtype, int metric, bool g, int threads, size_t smem, int minb = 3);
-uint32_t tier0_slots(const SearchPlan& p, uint32_t R);
 
 constexpr size_t kNoallocScratchBytes = PANN_NOALLOC_SCRATCH_BYTES;
 
@@ -202,38 +195,31 @@ extern "C" int pann_search_device_noalloc(pann_index* idx, const void* d_queries
   a.emu_count = cnt + 6;
 
   const size_t smem_cap = idx->smem_optin;
+  uint32_t wb2 = 0;
   // ---- first tier: shared-memory seen tables, no spill table, no hand-off
   {
-    uint32_t S = tier0_slots(plan, idx->R);
-    uint32_t wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, false);
-    int wpb = 4;
-    while (wpb > 1 && (size_t)wb * wpb > smem_cap) wpb >>= 1;
-    while ((size_t)wb * wpb > smem_cap && S > pow2_ceil(4ull * (idx->R + 1))) {
-      S >>= 1;
-      wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, false);
-    }
-    if ((size_t)wb * wpb > smem_cap) return fail(PANN_EINVAL, "search state for this beam does not fit in shared memory");
-    int occ = search_occupancy(idx->dtype, idx->metric, false, 32 * wpb, (size_t)wb * wpb);
-    if (occ <= 0) occ = 1;
-    uint64_t want = (nq + wpb - 1) / wpb;
-    int blocks = (int)std::min<uint64_t>(want, (uint64_t)occ * idx->sm_count);
+    TierSizes z;
+    rc = tier0_shape(idx, plan, nq, PREC_F32, 0, 0, 3, &z);
+    if (rc) return rc;
+    a.scr_bytes = search_scr_bytes(a.L, a.Ccap, z.scratch);
+    wb2 = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S2, SEEN_GLOBAL, z.scratch);
     SearchArgs t = a;
-    t.S = S;
-    t.warp_bytes = wb;
+    t.S = z.S;
+    t.id_bits = z.id_bits;
+    t.warp_bytes = z.wb;
     t.job_counter = cnt + 0;
     t.redo_list = redo0;
     t.redo_count = cnt + 3;
     t.gspill = nullptr;
     t.Sg = 0;
     t.inslog = nullptr;
-    PANN_CUDA(launch_search(idx->dtype, idx->metric, false, t, blocks, 32 * wpb, (size_t)wb * wpb, st, PREC_F32));
+    PANN_CUDA(launch_search(idx->dtype, idx->metric, z.seen, t, z.blocks, 32 * z.wpb, (size_t)z.wb * z.wpb, st, PREC_F32));
   }
   // ---- large-table tier: one global seen table per warp, in the scratch
   {
-    uint32_t wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S2, true);
     SearchArgs t = a;
     t.S = S2;
-    t.warp_bytes = wb;
+    t.warp_bytes = wb2;
     t.gtables = gt2;
     t.inslog = nullptr;
     t.job_list = redo0;
@@ -241,13 +227,13 @@ extern "C" int pann_search_device_noalloc(pann_index* idx, const void* d_queries
     t.job_counter = cnt + 2;
     t.redo_list = nullptr;
     t.redo_count = nullptr;
-    PANN_CUDA(launch_search(idx->dtype, idx->metric, true, t, t2_slots, 32, wb, st, PREC_F32));
+    PANN_CUDA(launch_search(idx->dtype, idx->metric, SEEN_GLOBAL, t, t2_slots, 32, wb2, st, PREC_F32));
   }
   // ---- emulation tiers: the reference's hashset emulated exactly, first in
   // shared memory, then (queries that outgrow it) in the scratch
   {
     uint32_t vs = pow2_ceil(8ull * plan.L + 64);
-    uint32_t basew = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, 0, true);
+    uint32_t basew = emu_state_bytes(idx->stride, plan.L, plan.Ccap, idx->R);
     SearchArgs t = a;
     t.redo_list = nullptr;
     t.redo_count = nullptr;

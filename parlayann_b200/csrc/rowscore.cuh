@@ -2,12 +2,16 @@
 //
 // Reading one row per lane costs the L1 a pass per lane and 16-byte chunk (32
 // rows of 384 bytes: 768 passes; tier 0 spent 85 % of its L1 pipe on them).
-// Here eight neighbouring lanes read the 128 contiguous bytes of a row, four
-// rows a load instruction, so the same rows cost 96 passes.
-//   8-bit: each lane multiplies its own chunks (integer sums are exact in any
-//          order) and eight partial sums are folded across the eight lanes
-//          with 7 shuffles, which leaves each lane one row's distance.
-//   float: the sum must run through a row in dimension order, so 32 rows x 128
+//   8-bit: four neighbouring lanes read 64 contiguous bytes of a row, eight
+//          rows a load instruction (a quarter of the passes); each lane
+//          multiplies its own chunks (integer sums are exact in any order) and
+//          four partial sums are folded across the four lanes with 3 shuffles,
+//          which leaves each lane one row's distance. Eight lanes a row halve
+//          the passes again but cost 30 more instructions, which a search
+//          waits for more than for the L1.
+//   float: eight lanes read 128 contiguous bytes, four rows an instruction (96
+//          passes for those 32 rows). The sum must run through a row in
+//          dimension order, so 32 rows x 128
 //          bytes pass through a 4 KB shared buffer per warp (cp.async, no
 //          registers held), chunk c of row r at slot c ^ (r % 8): both the
 //          8-lane writes and the per-lane reads of a row touch every bank
@@ -27,31 +31,37 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
 }
 
 // Lane l < n returns the distance of row `id` (its own) to the query staged at
-// qs (stage_query); n <= 32 rows, held by the first n lanes. Every lane of the
-// warp takes part; qs and stg are the warp's own.
+// qs (stage_query); 1 <= n <= 32 rows, held by the first n lanes (the other
+// lanes' ids are not used). Every lane of the warp takes part; qs and stg are the warp's own. Rows are at most 32 KB
+// (stride fits 32 bits).
 template <int DT, int MT>
-__device__ __forceinline__ float warp_score_rows(const uint8_t* __restrict__ points, uint64_t stride, int nchunks,
+__device__ __forceinline__ float warp_score_rows(const uint8_t* __restrict__ points, uint64_t stride64, int nchunks,
                                                  uint32_t id, int n, const uint8_t* qs, uint8_t* stg, int32_t qq,
                                                  int lane) {
   const unsigned FULL = 0xFFFFFFFFu;
-  const int g = lane >> 3, sub = lane & 7;
-  uint32_t rid[8];  // the rows this lane reads a part of: 4 j + g
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    rid[j] = __shfl_sync(FULL, id, 4 * j + g);
-    if (4 * j + g >= n) rid[j] = 0u;
-  }
-  const uint8_t* const base = points + 16 * sub;
+  const uint32_t stride = (uint32_t)stride64;
+  // loads that cover lanes past n repeat the first row (one fixed row instead, row 0, makes its L2 lines a hot spot
+  // for the whole device: 2.0 -> 2.3 ms for 10K queries of 96 floats)
+  const uint32_t id0 = __shfl_sync(FULL, id, 0);
+  if (lane >= n) id = id0;
   if (DT == DT_F32) {
+    const int g = lane >> 3, sub = lane & 7;
+    uint32_t rid[8];  // the rows this lane reads a part of: 4 j + g
+#pragma unroll
+    for (int j = 0; j < 8; j++) rid[j] = __shfl_sync(FULL, id, 4 * j + g);
     const float4* q = reinterpret_cast<const float4*>(qs);
-    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(stg);
+    // row 4 j + g's chunk goes to slot sub ^ (row % 8): two address patterns, j even and odd
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(stg) + 128u * g;
+    const uint32_t even = s0 + 16u * (sub ^ g), odd = s0 + 512u + 16u * (sub ^ (g + 4));
     auto issue = [&](int c0, int slot) {
       if (c0 + sub < nchunks) {
+        const uint8_t* const base = points + 16 * (c0 + sub);
+        const uint32_t de = even + 4096u * slot, dd = odd + 4096u * slot;
 #pragma unroll
-        for (int j = 0; j < 8; j++)
+        for (int j = 0; j < 8; j += 2)
           if (4 * j < n) {
-            const int r = 4 * j + g;
-            cp_async_16(sbase + 4096u * slot + 16u * (r * 8 + (sub ^ (r & 7))), base + rid[j] * stride + 16 * c0);
+            cp_async_16(de + 512u * j, base + (uint64_t)rid[j] * stride);
+            cp_async_16(dd + 512u * j, base + (uint64_t)rid[j + 1] * stride);
           }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -76,43 +86,43 @@ __device__ __forceinline__ float warp_score_rows(const uint8_t* __restrict__ poi
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     return MT == MT_L2 ? r : -r;
   } else {
+    const int g = lane >> 2, sub = lane & 3;
     const uint4* q = reinterpret_cast<const uint4*>(qs);
-    int32_t s[8];  // |p|^2 - 2 p.q (Euclidean) or p.q, this lane's chunks
-#pragma unroll
-    for (int j = 0; j < 8; j++) s[j] = 0;
-    for (int c0 = 0; c0 < nchunks; c0 += 8) {
-      if (c0 + sub < nchunks) {
-        const uint4 qc = q[c0 + sub];
-        uint4 v[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          if (4 * j < n) v[j] = __ldg(reinterpret_cast<const uint4*>(base + rid[j] * stride + 16 * c0));
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          if (4 * j < n) {
-            int32_t pq = 0, pp = 0;
-            int_chunk<DT, MT>(v[j], qc, pq, pp);
-            s[j] += MT == MT_L2 ? pp - 2 * pq : pq;
-          }
-      }
-    }
-    // fold across the eight lanes of a group: lane sub keeps row 4 sub + g
-    const bool h4 = sub & 4, h2 = sub & 2, h1 = sub & 1;
-    int32_t t4[4], t2[2];
+    const uint4* row[4];  // this lane's part of row 8 j + g
+    int32_t s[4];         // |p|^2 - 2 p.q (Euclidean) or p.q, this lane's chunks
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int32_t mine = h4 ? s[j + 4] : s[j], other = h4 ? s[j] : s[j + 4];
-      t4[j] = mine + __shfl_xor_sync(FULL, other, 4);
+      const uint32_t rid = __shfl_sync(FULL, id, 8 * j + g);
+      row[j] = reinterpret_cast<const uint4*>(points + (uint64_t)rid * stride) + sub;
+      s[j] = 0;
     }
+    for (int c0 = 0; c0 < nchunks; c0 += 8) {
+      const bool h0 = c0 + sub < nchunks, h1 = c0 + 4 + sub < nchunks;
+      const uint4 z = make_uint4(0, 0, 0, 0);
+      uint4 v[8];
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int32_t mine = h2 ? t4[j + 2] : t4[j], other = h2 ? t4[j] : t4[j + 2];
-      t2[j] = mine + __shfl_xor_sync(FULL, other, 2);
+      for (int j = 0; j < 4; j++)
+        if (8 * j < n) {
+          v[2 * j] = h0 ? __ldg(row[j] + c0) : z;
+          v[2 * j + 1] = h1 ? __ldg(row[j] + c0 + 4) : z;
+        }
+      const uint4 q0 = h0 ? q[c0 + sub] : z, q1 = h1 ? q[c0 + 4 + sub] : z;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (8 * j < n) {
+          int32_t pq = 0, pp = 0;
+          int_chunk<DT, MT>(v[2 * j], q0, pq, pp);
+          int_chunk<DT, MT>(v[2 * j + 1], q1, pq, pp);
+          s[j] += MT == MT_L2 ? pp - 2 * pq : pq;
+        }
     }
-    const int32_t mine = h1 ? t2[1] : t2[0], other = h1 ? t2[0] : t2[1];
-    int32_t tot = mine + __shfl_xor_sync(FULL, other, 1);
-    // row l = 4 sub' + g' sits at lane 8 g' + sub'
-    tot = __shfl_sync(FULL, tot, ((lane & 3) << 3) | (lane >> 2));
+    // fold across the four lanes of a group: lane sub keeps row 8 sub + g
+    const bool b1 = sub & 2, b0 = sub & 1;
+    const int32_t x0 = (b1 ? s[2] : s[0]) + __shfl_xor_sync(FULL, b1 ? s[0] : s[2], 2);
+    const int32_t x1 = (b1 ? s[3] : s[1]) + __shfl_xor_sync(FULL, b1 ? s[1] : s[3], 2);
+    int32_t tot = (b0 ? x1 : x0) + __shfl_xor_sync(FULL, b0 ? x0 : x1, 1);
+    // row l = 8 sub' + g' sits at lane 4 g' + sub'
+    tot = __shfl_sync(FULL, tot, ((lane & 7) << 2) | (lane >> 3));
     return MT == MT_L2 ? __int2float_rn(qq + tot) : -__int2float_rn(tot);
   }
 }

@@ -12,8 +12,10 @@ namespace pann {
 struct TierSizes {
   // tier 0: shared-memory seen tables, per-warp global spill tables
   uint32_t S = 0, wb = 0, Sg = 0;
+  int seen = SEEN32;     // entry width of the shared table
+  uint32_t id_bits = 0, scratch = 0;
   int wpb = 0, blocks = 0;
-  int minb = 3;      // resident blocks the first tier's registers are fitted to (3 or 4)
+  int minb = 3;      // the first tier's register budget (3: four resident blocks, 4: six)
   bool cta = false;  // every query on one block of the exact-emulation kernel instead of the first tiers
   size_t slots = 0, spill_bytes = 0;
   // hand-off from tier 0 to the emulation tier
@@ -46,7 +48,7 @@ struct TierBufs {
   const uint32_t* njobs0 = nullptr;     // optional tier-0 job count in device memory
 };
 
-cudaError_t launch_search(int dtype, int metric, bool global_table, const SearchArgs& a, int blocks, int threads,
+cudaError_t launch_search(int dtype, int metric, int seen, const SearchArgs& a, int blocks, int threads,
                           size_t smem, cudaStream_t st, int prec, int minb = 3);
 cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
                            int blocks, size_t smem, cudaStream_t st);
@@ -54,7 +56,9 @@ cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const Search
 constexpr int EMU_BLOCK_WARPS = 4;
 cudaError_t launch_emulate_block(int dtype, int metric, const SearchArgs& a, const EmuArgs& e, int blocks, size_t smem,
                                  cudaStream_t st);
-int search_occupancy(int dtype, int metric, bool g, int threads, size_t smem, int minb = 3);
+// Tier 0's table, warps and blocks (S_force, wpb_force: 0 = automatic).
+int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
+                int wpb_force, int minb, TierSizes* z);
 uint32_t tier0_slots(const SearchPlan& p, uint32_t R);
 
 // S_force / wpb_force (0 = automatic) override the tier-0 seen-table slots and

@@ -1,0 +1,64 @@
+"""The first search tier's row scoring (csrc/rowscore.cuh) and seen tables (csrc/search.cuh) at the ends of their
+blocks, against the oracle: ids, distances, visited and comparison counts bit for bit."""
+import numpy as np
+import pytest
+
+import parlayann_b200 as P
+from conftest import random_points
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def check(r, o):
+    np.testing.assert_array_equal(r.ids, o["ids"])
+    np.testing.assert_array_equal(r.dists, o["dists"])
+    np.testing.assert_array_equal(r.visited, o["visited"])
+    np.testing.assert_array_equal(r.cmps, o["cmps"])
+
+
+# rows of a part of a 16-byte chunk up to several 128-byte column blocks and a remainder; degrees that leave rounds of
+# 1 to 32 rows
+@pytest.mark.parametrize("d", [1, 4, 15, 16, 17, 31, 32, 33, 64, 65, 96, 127, 129, 300])
+@pytest.mark.parametrize("dtype,metric", [(np.uint8, P.L2), (np.int8, P.L2), (np.int8, P.MIPS), (np.float32, P.L2),
+                                          (np.float32, P.MIPS)])
+def test_row_lengths(d, dtype, metric, lib_built):
+    n, R = 1500, 37
+    base = random_points(dtype, n, d, d)
+    q = random_points(dtype, 40, d, d + 1)
+    g = O.random_graph(n, R, d + 2, min_deg=1)
+    idx = P.Index(base, R, metric)
+    idx.set_graph(g)
+    check(idx.search(q, 5, 24), O.search("oracle", base, q, g, 5, 24, metric=metric))
+    idx.close()
+
+
+# (points, degree, slots): 16-bit tables with distances of up to 2, 30 and 510 buckets from home, tables that fill and
+# spill, ids too wide for 16 bits (32-bit entries); beams whose frontier ends inside, at and past 32-entry words
+@pytest.mark.parametrize("n,R,slots", [(200_000, 16, 128), (200_000, 16, 2048), (5000, 16, 128), (900, 8, 4096),
+                                       (300_000, 16, 128)])
+@pytest.mark.parametrize("L", [10, 32, 33, 150])
+def test_seen_tables(n, R, slots, L, lib_built):
+    base = random_points(np.uint8, n, 8, 3)
+    q = random_points(np.uint8, 60, 8, 4)
+    g = O.random_graph(n, R, 5, min_deg=R // 2)
+    idx = P.Index(base, R)
+    idx.set_graph(g)
+    b = idx.batch(60, 10, L, seen_slots=slots)
+    check(b.run(q, 10, L), O.search("oracle", base, q, g, 10, L))
+    b.close()
+    check(idx.search(q, 10, L), O.search("oracle", base, q, g, 10, L))
+    idx.close()
+
+
+def test_long_frontier(lib_built):
+    """Frontiers past 1,024 entries (the unvisited flags no longer fit a warp's registers) and merges of more than 32
+    candidates."""
+    base = random_points(np.float32, 6000, 12, 7)
+    q = random_points(np.float32, 8, 12, 8)
+    g = O.random_graph(6000, 48, 9, min_deg=30)
+    idx = P.Index(base, 48)
+    idx.set_graph(g)
+    for L in (1000, 1024, 1100):
+        check(idx.search(q, 10, L), O.search("oracle", base, q, g, 10, L))
+    idx.close()
