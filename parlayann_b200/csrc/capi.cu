@@ -441,9 +441,10 @@ int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int p
 }
 
 int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArgs& a0, const TierSizes& z,
-                  const TierBufs& b, cudaStream_t st, int precision, uint32_t rerank, cudaStream_t side) {
+                  const TierBufs& b, cudaStream_t st, int precision, uint32_t rerank, cudaStream_t side, int phase) {
   uint32_t* cnt = b.cnt;
-  PANN_CUDA(cudaMemsetAsync(cnt, 0, 64, st));
+  if (phase & TIERS_FIRST) PANN_CUDA(cudaMemsetAsync(cnt, 0, 64, st));
+  if (!((phase & TIERS_FIRST) && (phase & TIERS_REST))) side = nullptr;
   // an emulation pass beside tier 0's tail: its blocks need most of an SM's
   // shared memory, so they start only as tier 0's blocks leave the SMs
   const bool early = side && idx->ev_fork && idx->ev_join && precision == PREC_F32 && z.emu_smem && !z.cta;
@@ -536,8 +537,10 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
                                emu_smem_bytes(z.base, z.vs, 0, 0, false), st));
       return PANN_OK;
     }
-    PANN_CUDA(launch_search(idx->dtype, idx->metric, z.seen, t, z.blocks, 32 * z.wpb, (size_t)z.wb * z.wpb, st, precision,
-                            z.minb));
+    if (phase & TIERS_FIRST)
+      PANN_CUDA(launch_search(idx->dtype, idx->metric, z.seen, t, z.blocks, 32 * z.wpb, (size_t)z.wb * z.wpb, st,
+                              precision, z.minb));
+    if (!(phase & TIERS_REST)) return PANN_OK;
   }
   if (early) {
     SearchArgs t = a;
@@ -711,7 +714,7 @@ static cudaStream_t side_stream(pann_index* idx) {
 int run_search(pann_index* idx, const SearchPlan& plan, const uint8_t* d_queries, const uint32_t* d_self_ids,
                uint32_t nq, const uint32_t* d_starts, uint32_t* d_ids, float* d_dists, uint32_t* d_vis,
                uint32_t* d_cmps, uint32_t* d_status, uint64_t* d_vis_keys, uint32_t vis_cap, cudaStream_t st,
-               int precision, uint32_t rerank, uint32_t parents, uint32_t scorer) {
+               int precision, uint32_t rerank, uint32_t parents, uint32_t scorer, int phase) {
   if (nq == 0) return PANN_OK;
   if (precision != PREC_F32 && idx->lp_prec != precision)
     return fail(PANN_EINVAL, "pann_index_set_precision was not called for this precision");
@@ -743,7 +746,7 @@ int run_search(pann_index* idx, const SearchPlan& plan, const uint8_t* d_queries
     if (rc) return rc;
     b.job_list0 = order;
   }
-  return enqueue_tiers(idx, plan, a, z, b, st, precision, rerank, side_stream(idx));
+  return enqueue_tiers(idx, plan, a, z, b, st, precision, rerank, side_stream(idx), phase);
 }
 
 int index_tier_buffers(pann_index* idx, const TierSizes& z, uint32_t nq, int precision, TierBufs* out) {
@@ -805,6 +808,29 @@ int stage_starts(pann_index* idx, const uint32_t* starts, uint32_t n_start, cuda
   } else {
     idx->starts_cached_n = 0;
   }
+  return PANN_OK;
+}
+
+// The per-query counts [visits nq][comparisons nq][status nq] (and one more word, if asked) at d to the host; waits
+// for the stream. One copy up to 256 KB (see pann_search).
+int copy_counts(const uint32_t* d, uint32_t nq, uint32_t* out_visited, uint32_t* out_cmps, uint32_t* status,
+                uint32_t* extra, cudaStream_t st) {
+  const size_t m = nq, words = 3 * m + (extra ? 1 : 0);
+  if (words <= 65536) {
+    std::vector<uint32_t> h(words);
+    PANN_CUDA(cudaMemcpyAsync(h.data(), d, 4 * words, cudaMemcpyDeviceToHost, st));
+    PANN_CUDA(cudaStreamSynchronize(st));
+    if (out_visited) std::memcpy(out_visited, h.data(), 4 * m);
+    if (out_cmps) std::memcpy(out_cmps, h.data() + m, 4 * m);
+    std::memcpy(status, h.data() + 2 * m, 4 * m);
+    if (extra) *extra = h[3 * m];
+    return PANN_OK;
+  }
+  if (out_visited) PANN_CUDA(cudaMemcpyAsync(out_visited, d, 4 * m, cudaMemcpyDeviceToHost, st));
+  if (out_cmps) PANN_CUDA(cudaMemcpyAsync(out_cmps, d + m, 4 * m, cudaMemcpyDeviceToHost, st));
+  PANN_CUDA(cudaMemcpyAsync(status, d + 2 * m, 4 * m, cudaMemcpyDeviceToHost, st));
+  if (extra) PANN_CUDA(cudaMemcpyAsync(extra, d + 3 * m, 4, cudaMemcpyDeviceToHost, st));
+  PANN_CUDA(cudaStreamSynchronize(st));
   return PANN_OK;
 }
 
@@ -1039,26 +1065,53 @@ int pann_search(pann_index* idx, const void* queries, uint32_t nq, const pann_qu
   const size_t k = plan.k;
   size_t rb = (size_t)idx->d * idx->esize;
   PANN_CUDA(idx->q.ensure(idx->stride * (size_t)nq));
-  PANN_CUDA(idx->ids.ensure(4 * std::max<size_t>(1, k * nq)));
-  PANN_CUDA(idx->dists.ensure(4 * std::max<size_t>(1, k * nq)));
-  PANN_CUDA(idx->vis.ensure(4 * (size_t)nq));
-  PANN_CUDA(idx->cmps.ensure(4 * (size_t)nq));
-  PANN_CUDA(idx->status.ensure(4 * (size_t)nq));
+  // ids, distances, visits, comparisons, status and the tiers' counters, one after another: small results come back
+  // in one copy (a copy into pageable memory costs 11 us however small: five of them were a third of a single
+  // query's time; past 256 KB the second copy on the host outweighs that)
+  const size_t rows = k * nq, words = 2 * rows + 3ull * nq;
+  PANN_CUDA(idx->ids.ensure(4 * (words + 16)));
+  uint32_t* d_ids = idx->ids.as<uint32_t>();
+  float* d_dists = reinterpret_cast<float*>(d_ids + rows);
+  uint32_t *d_vis = d_ids + 2 * rows, *d_cmps = d_vis + nq, *d_status = d_cmps + nq, *d_cnt = d_status + nq;
   if (rb != idx->stride) PANN_CUDA(cudaMemsetAsync(idx->q.p, 0, idx->stride * (size_t)nq, st));
   PANN_CUDA(cudaMemcpy2DAsync(idx->q.p, idx->stride, queries, rb, rb, nq, cudaMemcpyHostToDevice, st));
-  rc = run_search(idx, plan, idx->q.as<uint8_t>(), nullptr, nq, idx->starts.as<uint32_t>(), idx->ids.as<uint32_t>(),
-                  idx->dists.as<float>(), idx->vis.as<uint32_t>(), idx->cmps.as<uint32_t>(),
-                  idx->status.as<uint32_t>(), nullptr, 0, st);
+  auto run = [&](int phase) {
+    return run_search(idx, plan, idx->q.as<uint8_t>(), nullptr, nq, idx->starts.as<uint32_t>(), d_ids, d_dists, d_vis,
+                      d_cmps, d_status, nullptr, 0, st, 0, 0, 0, 0, phase);
+  };
+  if (words <= 65536) {
+    // few queries seldom need the later tiers: they are launched only if the first one's counters ask for them
+    // (four launches of about 4 us each behind a single query's search)
+    const bool first_only = nq <= 64;
+    std::vector<uint32_t> h(words + 16);
+    rc = run(first_only ? TIERS_FIRST : TIERS_ALL);
+    if (rc) return rc;
+    if (first_only) PANN_CUDA(cudaMemcpyAsync(d_cnt, idx->counters.p, 64, cudaMemcpyDeviceToDevice, st));
+    PANN_CUDA(cudaMemcpyAsync(h.data(), d_ids, 4 * (words + (first_only ? 16 : 0)), cudaMemcpyDeviceToHost, st));
+    PANN_CUDA(cudaStreamSynchronize(st));
+    if (first_only && (h[words + 3] | h[words + 6])) {  // queries to redo or to emulate
+      rc = run(TIERS_REST);
+      if (rc) return rc;
+      PANN_CUDA(cudaMemcpyAsync(h.data(), d_ids, 4 * words, cudaMemcpyDeviceToHost, st));
+      PANN_CUDA(cudaStreamSynchronize(st));
+    }
+    if (k) {
+      std::memcpy(out_ids, h.data(), 4 * rows);
+      if (out_dists) std::memcpy(out_dists, h.data() + rows, 4 * rows);
+    }
+    if (out_visited) std::memcpy(out_visited, h.data() + 2 * rows, 4ull * nq);
+    if (out_cmps) std::memcpy(out_cmps, h.data() + 2 * rows + nq, 4ull * nq);
+    return summarize_status(h.data() + 2 * rows + 2 * nq, nq, out_flags);
+  }
+  rc = run(TIERS_ALL);
   if (rc) return rc;
   if (k) {
-    PANN_CUDA(cudaMemcpyAsync(out_ids, idx->ids.p, 4 * k * nq, cudaMemcpyDeviceToHost, st));
-    if (out_dists) PANN_CUDA(cudaMemcpyAsync(out_dists, idx->dists.p, 4 * k * nq, cudaMemcpyDeviceToHost, st));
+    PANN_CUDA(cudaMemcpyAsync(out_ids, d_ids, 4 * rows, cudaMemcpyDeviceToHost, st));
+    if (out_dists) PANN_CUDA(cudaMemcpyAsync(out_dists, d_dists, 4 * rows, cudaMemcpyDeviceToHost, st));
   }
-  if (out_visited) PANN_CUDA(cudaMemcpyAsync(out_visited, idx->vis.p, 4 * (size_t)nq, cudaMemcpyDeviceToHost, st));
-  if (out_cmps) PANN_CUDA(cudaMemcpyAsync(out_cmps, idx->cmps.p, 4 * (size_t)nq, cudaMemcpyDeviceToHost, st));
   std::vector<uint32_t> status(nq);
-  PANN_CUDA(cudaMemcpyAsync(status.data(), idx->status.p, 4 * (size_t)nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaStreamSynchronize(st));
+  int crc = copy_counts(d_vis, nq, out_visited, out_cmps, status.data(), nullptr, st);
+  if (crc) return crc;
   return summarize_status(status.data(), nq, out_flags);
 }
 

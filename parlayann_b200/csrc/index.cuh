@@ -109,6 +109,9 @@ struct SearchPlan {
   uint32_t Ccap;
 };
 
+// Which tiers a call enqueues (tiers.cuh).
+enum : int { TIERS_FIRST = 1, TIERS_REST = 2, TIERS_ALL = 3 };
+
 int make_plan(const pann_index* idx, const pann_query_params* qp, uint32_t n_start, SearchPlan* plan);
 
 // Run the tiered search on device buffers (queries already in index row layout).
@@ -118,7 +121,7 @@ int make_plan(const pann_index* idx, const pann_query_params* qp, uint32_t n_sta
 int run_search(pann_index* idx, const SearchPlan& plan, const uint8_t* d_queries, const uint32_t* d_self_ids,
                uint32_t nq, const uint32_t* d_starts, uint32_t* d_ids, float* d_dists, uint32_t* d_vis,
                uint32_t* d_cmps, uint32_t* d_status, uint64_t* d_vis_keys, uint32_t vis_cap, cudaStream_t st,
-               int precision = 0, uint32_t rerank = 0, uint32_t parents = 0, uint32_t scorer = 0);
+               int precision = 0, uint32_t rerank = 0, uint32_t parents = 0, uint32_t scorer = 0, int phase = TIERS_ALL);
 
 // A batch laid out in a caller's device arena (the serving form's admission
 // by scratch memory): every buffer of one run of nq queries, whose k and beam

@@ -312,12 +312,12 @@ extern "C" int pann_search_quantized(pann_index* idx, const void* queries, uint3
   PANN_CUDA(qi->q.ensure(qi->stride * (size_t)nq));
   PANN_CUDA(qi->ids.ensure(4ull * kp * nq));
   PANN_CUDA(qi->dists.ensure(4ull * kp * nq));
-  PANN_CUDA(qi->vis.ensure(4ull * nq));
-  PANN_CUDA(qi->cmps.ensure(4ull * nq));
-  PANN_CUDA(qi->status.ensure(4ull * nq));
-  PANN_CUDA(idx->ids.ensure(4ull * qp->k * nq));
-  PANN_CUDA(idx->dists.ensure(4ull * qp->k * nq));
-  PANN_CUDA(idx->counters.ensure(16));
+  // results, then visits, comparisons, status and the count of short answers, one after another
+  const size_t rows = (size_t)qp->k * nq;
+  PANN_CUDA(idx->ids.ensure(4 * (2 * rows + 3ull * nq + 4)));
+  uint32_t* d_ids = idx->ids.as<uint32_t>();
+  float* d_dists = reinterpret_cast<float*>(d_ids + rows);
+  uint32_t *d_vis = d_ids + 2 * rows, *short_count = d_vis + 3ull * nq;
   if (rb != idx->stride) PANN_CUDA(cudaMemsetAsync(idx->q.p, 0, idx->stride * (size_t)nq, st));
   PANN_CUDA(cudaMemcpy2DAsync(idx->q.p, idx->stride, queries, rb, rb, nq, cudaMemcpyHostToDevice, st));
   {  // the queries, translated as the points were
@@ -332,28 +332,22 @@ extern "C" int pann_search_quantized(pann_index* idx, const void* queries, uint3
     PANN_CUDA(cudaGetLastError());
   }
   rc = run_search(qi, plan, qi->q.as<uint8_t>(), nullptr, nq, qi->starts.as<uint32_t>(), qi->ids.as<uint32_t>(),
-                  qi->dists.as<float>(), qi->vis.as<uint32_t>(), qi->cmps.as<uint32_t>(), qi->status.as<uint32_t>(),
-                  nullptr, 0, st);
+                  qi->dists.as<float>(), d_vis, d_vis + nq, d_vis + 2ull * nq, nullptr, 0, st);
   if (rc) return rc;
-  uint32_t* short_count = idx->counters.as<uint32_t>();
   PANN_CUDA(cudaMemsetAsync(short_count, 0, 4, st));
   {
     auto kern = idx->metric == PANN_MIPS ? quant_rerank_kernel<MT_IP> : quant_rerank_kernel<MT_L2>;
     PANN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max()));
     kern<<<(nq + 3) / 4, 128, smem, st>>>(idx->d_points, idx->stride, idx->d, idx->nchunks, idx->q.as<uint8_t>(), nq,
-                                          qi->ids.as<uint32_t>(), kp, qp->k, idx->ids.as<uint32_t>(),
-                                          idx->dists.as<float>(), short_count);
+                                          qi->ids.as<uint32_t>(), kp, qp->k, d_ids, d_dists, short_count);
     PANN_CUDA(cudaGetLastError());
   }
   std::vector<uint32_t> status(nq);
   uint32_t h_short = 0;
-  PANN_CUDA(cudaMemcpyAsync(out_ids, idx->ids.p, 4ull * qp->k * nq, cudaMemcpyDeviceToHost, st));
-  if (out_dists) PANN_CUDA(cudaMemcpyAsync(out_dists, idx->dists.p, 4ull * qp->k * nq, cudaMemcpyDeviceToHost, st));
-  if (out_visited) PANN_CUDA(cudaMemcpyAsync(out_visited, qi->vis.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  if (out_cmps) PANN_CUDA(cudaMemcpyAsync(out_cmps, qi->cmps.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(status.data(), qi->status.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(&h_short, short_count, 4, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaStreamSynchronize(st));
+  PANN_CUDA(cudaMemcpyAsync(out_ids, d_ids, 4 * rows, cudaMemcpyDeviceToHost, st));
+  if (out_dists) PANN_CUDA(cudaMemcpyAsync(out_dists, d_dists, 4 * rows, cudaMemcpyDeviceToHost, st));
+  rc = copy_counts(d_vis, nq, out_visited, out_cmps, status.data(), &h_short, st);
+  if (rc) return rc;
   for (uint32_t i = 0; i < nq; i++)
     if (status[i] & (QS_TABLE_FULL | QS_INTERNAL)) return fail(PANN_EOVERFLOW, "a query's seen-set outgrew the largest table");
   if (h_short) return fail(PANN_ESHORT, "beam search returned fewer than k results");

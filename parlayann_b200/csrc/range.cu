@@ -445,9 +445,8 @@ extern "C" int pann_range_search(pann_index* idx, const void* queries, uint32_t 
   PANN_CUDA(idx->q.ensure_grow(idx->stride * (size_t)nq));
   PANN_CUDA(idx->ids.ensure_grow(4ull * beam * nq));
   PANN_CUDA(idx->dists.ensure_grow(4ull * beam * nq));
-  PANN_CUDA(idx->vis.ensure_grow(4ull * nq));
-  PANN_CUDA(idx->cmps.ensure_grow(4ull * nq));
-  PANN_CUDA(idx->status.ensure_grow(4ull * nq));
+  PANN_CUDA(idx->vis.ensure_grow(12ull * nq));  // visits, comparisons, status
+  uint32_t* d_vis = idx->vis.as<uint32_t>();
   if (rb != idx->stride) PANN_CUDA(cudaMemsetAsync(idx->q.p, 0, idx->stride * (size_t)nq, st));
   PANN_CUDA(cudaMemcpy2DAsync(idx->q.p, idx->stride, queries, rb, rb, nq, cudaMemcpyHostToDevice, st));
 
@@ -465,8 +464,8 @@ extern "C" int pann_range_search(pann_index* idx, const void* queries, uint32_t 
     rc = index_tier_buffers(idx, z, nq, PREC_F32, &b);
     if (rc) return rc;
     SearchArgs a = base_args(idx, plan, idx->q.as<uint8_t>(), nullptr, nq, idx->starts.as<uint32_t>(),
-                             idx->ids.as<uint32_t>(), idx->dists.as<float>(), idx->vis.as<uint32_t>(),
-                             idx->cmps.as<uint32_t>(), idx->status.as<uint32_t>(), nullptr, 0);
+                             idx->ids.as<uint32_t>(), idx->dists.as<float>(), d_vis, d_vis + nq, d_vis + 2ull * nq,
+                             nullptr, 0);
     a.es_count = (double)rp->early_stopping_count;
     a.es_radius = rp->type == PANN_RANGE_DOUBLING ? rp->radius : r_f;
     a.es_esr = esr_f;
@@ -586,17 +585,15 @@ extern "C" int pann_range_search(pann_index* idx, const void* queries, uint32_t 
   }
 
   // ---- 4. counts, offsets, the CSR gather
-  std::vector<uint32_t> h_n(nq), h_src(nq), h_extra(nq), h_rst(nq), h_rcmps(nq), h_vis(nq), h_cmps(nq), h_st(nq);
+  // res_n, src, extra, rstat and rcmps lie one after another, as do the search's three counts: two copies
+  std::vector<uint32_t> h_meta(5ull * nq), h_search(3ull * nq);
   PANN_CUDA(cudaStreamSynchronize(st));
-  PANN_CUDA(cudaMemcpyAsync(h_n.data(), res_n, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_src.data(), src, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_extra.data(), extra, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_rst.data(), rstat, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_rcmps.data(), rcmps, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_vis.data(), idx->vis.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_cmps.data(), idx->cmps.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
-  PANN_CUDA(cudaMemcpyAsync(h_st.data(), idx->status.p, 4ull * nq, cudaMemcpyDeviceToHost, st));
+  PANN_CUDA(cudaMemcpyAsync(h_meta.data(), res_n, 20ull * nq, cudaMemcpyDeviceToHost, st));
+  PANN_CUDA(cudaMemcpyAsync(h_search.data(), d_vis, 12ull * nq, cudaMemcpyDeviceToHost, st));
   PANN_CUDA(cudaStreamSynchronize(st));
+  const uint32_t *h_n = h_meta.data(), *h_src = h_n + nq, *h_extra = h_src + nq, *h_rst = h_extra + nq,
+                 *h_rcmps = h_rst + nq;
+  const uint32_t *h_vis = h_search.data(), *h_cmps = h_vis + nq, *h_st = h_cmps + nq;
   for (uint32_t i = 0; i < nq; i++) {
     if (h_st[i] & (QS_TABLE_FULL | QS_INTERNAL)) return fail(PANN_EOVERFLOW, "a query's seen-set outgrew the largest table");
     if (h_rst[i] & RS_RETRY) return fail(PANN_EOVERFLOW, "a range expansion outgrew the largest table");

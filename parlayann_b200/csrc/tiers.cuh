@@ -65,11 +65,14 @@ uint32_t tier0_slots(const SearchPlan& p, uint32_t R);
 // warps per block.
 int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
                int wpb_force, TierSizes* z, int minb_force = 0);
+// phase: the first tier, the tiers after it (on the first one's counters and
+// lists, untouched since), or both.
 // side (optional): the index's side stream; the exact-emulation tier then
 // also runs a pass beside tier 0's tail on it (idx->ev_fork / ev_join order
 // it), taking hand-offs as they are published without waiting for any.
 int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArgs& a, const TierSizes& z,
-                  const TierBufs& b, cudaStream_t st, int precision, uint32_t rerank, cudaStream_t side = nullptr);
+                  const TierBufs& b, cudaStream_t st, int precision, uint32_t rerank, cudaStream_t side = nullptr,
+                  int phase = TIERS_ALL);
 // The tier-0 job order farthest-from-the-start-point first (order.cu):
 // *order points into idx->order, valid until the next call.
 int order_far_first(pann_index* idx, const uint8_t* d_queries, const uint32_t* d_self_ids, const uint32_t* d_starts,
@@ -84,6 +87,8 @@ int order_batch(const pann_index* idx, const uint8_t* d_queries, const uint32_t*
 // tile_rows > 0 fixes the rows staged per round (CUDA-core scoring), else chosen for occupancy.
 int enqueue_tile(const pann_index* idx, const SearchPlan& plan, SearchArgs a, uint32_t parents, uint32_t* job_counter,
                  int precision, uint32_t rerank, cudaStream_t st, uint32_t scorer = 0, uint32_t tile_rows = 0);
+int copy_counts(const uint32_t* d, uint32_t nq, uint32_t* out_visited, uint32_t* out_cmps, uint32_t* status,
+                uint32_t* extra, cudaStream_t st);
 // Validates the start points and copies them to idx->starts (cached).
 int stage_starts(pann_index* idx, const uint32_t* starts, uint32_t n_start, cudaStream_t st);
 // The index's own tier buffers for nq queries (grown as needed).
