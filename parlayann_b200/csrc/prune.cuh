@@ -20,46 +20,109 @@ namespace pann {
 // Keys carry PANN_VFLAG while a candidate is not one of the row's clean
 // entries ("fresh").
 
-// Sort n keys (kin, flags ignored in the order, ties by position) into out,
-// dropping repeated ids (index.h:86-88); a repeat is fresh only if all copies
-// are. Warp-cooperative: every lane ranks up to eight keys a pass against
-// each key in turn. Returns the number of distinct keys.
-__device__ __forceinline__ uint32_t prune_sort_unique(uint64_t* kin, uint32_t n, uint64_t* out, int lane) {
-  const unsigned FULL = 0xFFFFFFFFu;
-  constexpr int K = 4;
-  for (uint32_t b = 0; b < n; b += 32 * K) {
-    uint64_t mk[K];
-    uint32_t r[K];
+// Bitonic sort of 32 KPL keys in registers, key i = lane * KPL + j.
+template <int KPL>
+__device__ __forceinline__ void warp_bitonic(uint64_t (&k)[KPL], int lane) {
 #pragma unroll
-    for (int q = 0; q < K; q++) {
-      const uint32_t i = b + 32 * q + lane;
-      mk[q] = i < n ? kin[i] & PANN_KEYMASK : ~0ull;
-      r[q] = 0;
-    }
-#pragma unroll 4
-    for (uint32_t j = 0; j < n; j++) {
-      const uint64_t kj = kin[j] & PANN_KEYMASK;
+  for (int size = 2; size <= 32 * KPL; size <<= 1) {
 #pragma unroll
-      for (int q = 0; q < K; q++) r[q] += (kj < mk[q]) | ((kj == mk[q]) & (j < b + 32 * q + lane));
-    }
+    for (int st = size >> 1; st > 0; st >>= 1) {
+      if (st >= KPL) {  // partner in another lane
+        const int ls = st / KPL;
+        const bool up = size >= 32 * KPL || ((lane * KPL) & size) == 0;
+        const bool low = (lane & ls) == 0;
 #pragma unroll
-    for (int q = 0; q < K; q++) {
-      const uint32_t i = b + 32 * q + lane;
-      if (i < n) out[r[q]] = kin[i];
+        for (int j = 0; j < KPL; j++) {
+          const uint64_t o = __shfl_xor_sync(0xFFFFFFFFu, k[j], ls);
+          k[j] = ((o < k[j]) == (low == up)) ? o : k[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < KPL; j++)
+          if ((j & st) == 0) {
+            const bool up = size >= KPL ? (size >= 32 * KPL || ((lane * KPL) & size) == 0) : (j & size) == 0;
+            const uint64_t x = k[j], y = k[j | st];
+            const bool sw = (y < x) == up;
+            k[j] = sw ? y : x;
+            k[j | st] = sw ? x : y;
+          }
+      }
     }
   }
+}
+
+// Sort the n <= 32 KPL keys of kin by (distance, id) in registers (1,300
+// instructions for 256 keys, a rank sort of 200 keys 6,800), drop repeated ids
+// (index.h:86-88; a repeat is fresh only if all copies are) and leave the
+// distinct keys in kin.
+template <int KPL>
+__device__ __forceinline__ uint32_t prune_sort_regs(uint64_t* kin, uint32_t n, int lane) {
+  const unsigned FULL = 0xFFFFFFFFu;
+  uint64_t k[KPL];
+  // the flag below the id: copies of an id end up next to each other, a clean one first
+#pragma unroll
+  for (int j = 0; j < KPL; j++) {
+    const uint32_t i = 32 * j + lane;
+    const uint64_t v = i < n ? kin[i] : ~0ull;
+    k[j] = i < n ? (v & 0xFFFFFFFF00000000ull) | ((uint32_t)v << 1) | (uint32_t)((v >> 31) & 1u) : ~0ull;
+  }
   __syncwarp();
-  // repeats are adjacent (equal ids carry equal distances)
+  warp_bitonic<KPL>(k, lane);
+  // the first of each id stays
+  const uint64_t prev = __shfl_up_sync(FULL, k[KPL - 1], 1);
+  bool keep[KPL];
+  uint32_t c = 0;
+#pragma unroll
+  for (int j = 0; j < KPL; j++) {
+    const uint64_t before = j ? k[j - 1] : prev;
+    const uint32_t i = lane * KPL + j;
+    keep[j] = i < n && (i == 0 || (uint32_t)(before >> 1) << 1 != (uint32_t)(k[j] >> 1) << 1);
+    c += keep[j];
+  }
+  uint32_t at = c;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, at, d);
+    if (lane >= d) at += t;
+  }
+  const uint32_t u = __shfl_sync(FULL, at, 31);
+  at -= c;
+#pragma unroll
+  for (int j = 0; j < KPL; j++)
+    if (keep[j]) {
+      const uint32_t lo = (uint32_t)k[j];
+      kin[at++] = (k[j] & 0xFFFFFFFF00000000ull) | (lo >> 1) | ((lo & 1u) << 31);
+    }
+  __syncwarp();
+  return u;
+}
+
+// As prune_sort_regs for any n, through `tmp` (n keys) past 512 keys.
+__device__ __forceinline__ uint32_t prune_sort_unique(uint64_t* kin, uint32_t n, uint64_t* tmp, int lane) {
+  if (n <= 128) return prune_sort_regs<4>(kin, n, lane);
+  if (n <= 256) return prune_sort_regs<8>(kin, n, lane);
+  if (n <= 512) return prune_sort_regs<16>(kin, n, lane);
+  const unsigned FULL = 0xFFFFFFFFu;
+  for (uint32_t i = lane; i < n; i += 32) {
+    const uint64_t ki = kin[i] & PANN_KEYMASK;
+    uint32_t r = 0;
+    for (uint32_t j = 0; j < n; j++) {
+      const uint64_t kj = kin[j] & PANN_KEYMASK;
+      r += (kj < ki) | ((kj == ki) & (j < i));
+    }
+    tmp[r] = kin[i];
+  }
+  __syncwarp();
   uint32_t u = 0;
   for (uint32_t b = 0; b < n; b += 32) {
     const uint32_t i = b + lane;
     uint64_t k = 0;
     bool first = false;
     if (i < n) {
-      k = out[i];
-      first = i == 0 || key_id(out[i - 1]) != key_id(k);
+      k = tmp[i];
+      first = i == 0 || key_id(tmp[i - 1]) != key_id(k);
       if (first)
-        for (uint32_t j = i + 1; j < n && key_id(out[j]) == key_id(k); j++) k &= out[j] | PANN_KEYMASK;
+        for (uint32_t j = i + 1; j < n && key_id(tmp[j]) == key_id(k); j++) k &= tmp[j] | PANN_KEYMASK;
     }
     const unsigned m = __ballot_sync(FULL, first);
     __syncwarp();

@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "index.cuh"
 #include "lowprec.cuh"
+#include "rowscore.cuh"
 #include "tiers.cuh"
 #include "umma.cuh"
 
@@ -48,7 +49,7 @@ __host__ __device__ inline TileLayout tile_layout(uint32_t d, uint32_t L, uint32
                                                   uint64_t lp_stride, uint32_t CWs, bool tc = false) {
   TileLayout t{};
   size_t o = 0;
-  const size_t dpad = (d + 3) & ~3u;
+  const size_t dpad = (d + 15) & ~15u;  // whole 16-byte chunks of the low-precision row, of either type
   // rows at an odd multiple of 16 bytes apart: conflict-free 16-byte reads
   t.sstride = (uint32_t)(((lp_stride / 16) % 2 == 0) ? lp_stride + 16 : lp_stride);
   // every region starts on a 16-byte boundary (cp.async destinations and MMA operands need it)
@@ -76,57 +77,65 @@ __host__ __device__ inline TileLayout tile_layout(uint32_t d, uint32_t L, uint32
   return t;
 }
 
-// Exact float32 distance in the reference's order (euclidian_point.h:83-90,
-// mips_point.h:60-66): sequential sum, every product and sum rounded on its own.
-template <int MT>
-__device__ __forceinline__ float exact_f32_dist(const float* __restrict__ row, const float* q, uint32_t d) {
-  float r = 0.0f;
-  for (uint32_t i = 0; i < d; i++) {
-    if (MT == MT_L2) {
-      const float t = __fsub_rn(__ldg(row + i), q[i]);
-      r = __fadd_rn(r, __fmul_rn(t, t));
-    } else {
-      r = __fadd_rn(r, __fmul_rn(__ldg(row + i), q[i]));
-    }
-  }
-  return MT == MT_L2 ? r : -r;
+__device__ __forceinline__ uint64_t fma2_rn(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 
-// Approximate distance of one staged low-precision row (16-byte reads).
-template <int MT, int PREC>
-__device__ __forceinline__ float tile_row_dist(const uint8_t* row, const float* q, const float* sc, uint32_t d,
-                                               uint32_t chunks) {
-  float a0 = 0.f, a1 = 0.f;
+// Approximate distance of one staged low-precision row (16-byte reads), two
+// neighbouring values at a time (paired FP32). q: the query; sc (FP8): the
+// per-dimension scales, negated for Euclidean distance (NEG: as stored), so that
+// one fused step gives q - x s; both zero-padded to whole 16-byte chunks of the row, whose
+// padding then adds nothing. Even and odd values have a sum each.
+template <int MT, int PREC, bool NEG>
+__device__ __forceinline__ float tile_row_dist(const uint8_t* row, const float* q, const float* sc, uint32_t chunks) {
+  uint64_t acc = 0;
+  const uint64_t minus_one = 0xBF800000BF800000ull;
   constexpr uint32_t VPC = PREC == PREC_BF16 ? 8 : 16;
   for (uint32_t c = 0; c < chunks; c++) {
     const uint4 v = reinterpret_cast<const uint4*>(row)[c];
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float4* q4 = reinterpret_cast<const float4*>(q + c * VPC);
+    const float4* s4 = reinterpret_cast<const float4*>(sc + c * VPC);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < (int)VPC / 4; j++) {  // four values
+      uint64_t x[2];
+      if (PREC == PREC_BF16) {
 #pragma unroll
-      for (int h = 0; h < (PREC == PREC_BF16 ? 1 : 2); h++) {
-        const uint32_t e = c * VPC + j * (VPC / 4) + 2 * h;
-        if (e >= d) break;
-        float2 x;
-        if (PREC == PREC_BF16) {
-          x = bf16x2_to_f2(w[j]);
-        } else {
-          x = e4m3x2_to_f2(w[j] >> (16 * h));
-          x.x *= sc[e];
-          x.y *= sc[e + 1];
+        for (int h = 0; h < 2; h++) {
+          const float2 f = bf16x2_to_f2(w[2 * j + h]);
+          x[h] = pk2(f.x, f.y);
         }
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const float2 f = e4m3x2_to_f2(w[j] >> (16 * h));
+          x[h] = pk2(f.x, f.y);
+        }
+      }
+      const float4 qv = q4[j];
+      const uint64_t qq[2] = {pk2(qv.x, qv.y), pk2(qv.z, qv.w)};
+      uint64_t ss[2] = {0, 0};
+      if (PREC == PREC_FP8) {
+        const float4 sv = s4[j];
+        const uint64_t flip = MT == MT_L2 && !NEG ? 0x8000000080000000ull : 0ull;
+        ss[0] = pk2(sv.x, sv.y) ^ flip;
+        ss[1] = pk2(sv.z, sv.w) ^ flip;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
         if (MT == MT_L2) {
-          const float t0 = x.x - q[e], t1 = x.y - q[e + 1];
-          a0 = fmaf(t0, t0, a0);
-          a1 = fmaf(t1, t1, a1);
+          const uint64_t t = fma2_rn(x[h], PREC == PREC_FP8 ? ss[h] : minus_one, qq[h]);
+          acc = fma2_rn(t, t, acc);
         } else {
-          a0 = fmaf(x.x, q[e], a0);
-          a1 = fmaf(x.y, q[e + 1], a1);
+          acc = fma2_rn(PREC == PREC_FP8 ? mul2_rn(x[h], ss[h]) : x[h], qq[h], acc);
         }
       }
     }
   }
-  return MT == MT_L2 ? a0 + a1 : -(a0 + a1);
+  const float r = __uint_as_float((uint32_t)acc) + __uint_as_float((uint32_t)(acc >> 32));
+  return MT == MT_L2 ? r : -r;
 }
 
 // Seen-set slots of a query with beam L: (L + 16) * nel * 1.35 rounded up to
@@ -165,7 +174,7 @@ constexpr uint64_t TC_WAIT_LIMIT = 1000000000ull;
 // row's squared norm precomputed (SearchArgs::lp_norms). The traversal, the
 // cutoff, the merge and the exact re-rank are those of the CUDA-core scoring.
 template <int MT, int PREC, bool TC>
-__global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t W, uint32_t S, uint32_t CW,
+__global__ void __launch_bounds__(128, 6) search_tile_kernel(SearchArgs a, uint32_t W, uint32_t S, uint32_t CW,
                                                           uint32_t CWs) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x;
@@ -186,8 +195,12 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
   //       [9] truncated
   uint32_t* par = misc + 5;
   const uint32_t nel = a.dl < a.R ? a.dl : a.R;
+  // the staged chunks this thread copies: (row, chunk) from here on in steps of blockDim.x chunks
+  const uint32_t tid_r = (uint32_t)tid / a.lp_chunks, tid_c = (uint32_t)tid % a.lp_chunks;
+  const uint32_t step_r = blockDim.x / a.lp_chunks, step_c = blockDim.x % a.lp_chunks;
   if (PREC == PREC_FP8)
-    for (uint32_t i = tid; i < a.d; i += blockDim.x) sc[i] = a.lp_scales[i];
+    for (uint32_t i = tid; i < ((a.d + 15) & ~15u); i += blockDim.x)
+      sc[i] = i >= a.d ? 0.0f : MT == MT_L2 && !TC ? -a.lp_scales[i] : a.lp_scales[i];
   const uint32_t njobs = a.njobs_dev ? *a.njobs_dev : a.nq;
   // tensor-core state: the MMA barrier, the tensor-memory columns (32, of
   // which the 16 of N are used), the barrier's phase
@@ -215,7 +228,7 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
     const uint32_t Sq = a.qL ? tile_seen_slots(L, nel, a.R) : S;  // <= S
     const uint32_t fill_limit = Sq - Sq / 16;
     const float* qsrc = reinterpret_cast<const float*>(a.queries + (uint64_t)qi * a.stride);
-    for (uint32_t i = tid; i < a.d; i += blockDim.x) qf[i] = qsrc[i];
+    for (uint32_t i = tid; i < ((a.d + 15) & ~15u); i += blockDim.x) qf[i] = i < a.d ? qsrc[i] : 0.0f;
     for (uint32_t i = tid; i < Sq; i += blockDim.x) table[i] = PANN_PAD;
     if (tid < 15) misc[1 + tid] = 0;
     __syncthreads();
@@ -273,7 +286,7 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
     // start points: approximate distances from global rows, all in the seen set
     for (uint32_t s = tid; s < a.n_start; s += blockDim.x) {
       const uint32_t id = a.starts[s];
-      const float dd = tile_row_dist<MT, PREC>(a.lp_rows + (uint64_t)id * a.lp_stride, qf, sc, a.d, a.lp_chunks);
+      const float dd = tile_row_dist<MT, PREC, !TC>(a.lp_rows + (uint64_t)id * a.lp_stride, qf, sc, a.lp_chunks);
       cand[s] = make_key(dd, id);
       uint32_t h = tile_slot(id, Sq);
       for (uint32_t p = 0; p < Sq; p++) {
@@ -334,32 +347,48 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
       const uint32_t np = misc[3];
       if (np == 0) break;
       nvis += np;
-      // ---- adjacency rows of the parents; new neighbours into the tile
-      for (uint32_t x = tid; x < np * nel; x += blockDim.x) {
-        const uint32_t p = x / nel, j = x - p * nel;
-        const uint32_t id = a.graph[(uint64_t)par[p] * a.R + j];
-        if (id == PANN_PAD) continue;
-        uint32_t h = tile_slot(id, Sq);
-        for (uint32_t probe = 0; probe < Sq; probe++) {
-          const uint32_t old = atomicCAS(table + h, PANN_PAD, id);
-          if (old == id) break;
-          if (old == PANN_PAD) {
-            const uint32_t e = atomicAdd(misc + 4, 1u);
-            if (e >= fill_limit) misc[9] = 1;  // stop after this step: the table is nearly full
-            cid[atomicAdd(misc + 1, 1u)] = id;
-            break;
-          }
-          h = h + 1 == Sq ? 0 : h + 1;
+      // ---- adjacency rows of the parents; new neighbours into the tile (a warp's new ids take one counter step)
+      for (uint32_t x0 = 32 * warp; x0 < np * nel; x0 += blockDim.x) {
+        const uint32_t x = x0 + lane;
+        uint32_t id = PANN_PAD;
+        if (x < np * nel) {
+          const uint32_t p = (x >= nel) + (x >= 2 * nel) + (x >= 3 * nel);
+          id = __ldg(a.graph + (uint64_t)par[p] * a.R + (x - p * nel));
         }
+        bool fresh = false;
+        if (id != PANN_PAD) {
+          uint32_t h = tile_slot(id, Sq);
+          for (uint32_t probe = 0; probe < Sq; probe++) {
+            const uint32_t old = atomicCAS(table + h, PANN_PAD, id);
+            if (old == id) break;
+            if (old == PANN_PAD) {
+              fresh = true;
+              break;
+            }
+            h = h + 1 == Sq ? 0 : h + 1;
+          }
+        }
+        const unsigned m = __ballot_sync(FULL, fresh);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(misc + 1, (uint32_t)__popc(m));
+        at = __shfl_sync(FULL, at, 0);
+        if (fresh) cid[at + __popc(m & ((1u << lane) - 1u))] = id;
       }
       __syncthreads();
       const uint32_t ncand = misc[1];
+      if (tid == 0) {
+        misc[4] += ncand;
+        if (misc[4] > fill_limit) misc[9] = 1;  // stop after this step: the table is nearly full
+      }
       const float cutoff = fn == L ? key_dist(fr[L - 1]) : 3.40282346638528859812e+38F;
       for (uint32_t c0 = 0; c0 < ncand && tc_ok; c0 += CWs) {
         const uint32_t nr = ncand - c0 < CWs ? ncand - c0 : CWs;
         // ---- stage the tile's rows (one round trip per CWs rows)
-        for (uint32_t x = tid; x < nr * a.lp_chunks; x += blockDim.x) {
-          const uint32_t r = x / a.lp_chunks, c = x - r * a.lp_chunks;
+        for (uint32_t r = tid_r, c = tid_c; r < nr; r += step_r, c += step_c) {
+          if (c >= a.lp_chunks) {
+            c -= a.lp_chunks;
+            if (++r >= nr) break;
+          }
           const uint32_t off = TC ? cm_offset(r, c, a.lp_chunks) : r * ly.sstride + 16 * c;
           cp_async16(stage + off, a.lp_rows + (uint64_t)cid[c0 + r] * a.lp_stride + 16 * c);
         }
@@ -401,9 +430,16 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
         } else {
           __syncthreads();
           // ---- score; keep those below the cutoff of a full frontier (beamSearch.h:173-182)
-          for (uint32_t r = tid; r < nr; r += blockDim.x) {
-            const float dd = tile_row_dist<MT, PREC>(stage + (size_t)r * ly.sstride, qf, sc, a.d, a.lp_chunks);
-            if (dd < cutoff) cand[atomicAdd(misc + 2, 1u)] = make_key(dd, cid[c0 + r]);
+          for (uint32_t r0 = 32 * warp; r0 < nr; r0 += blockDim.x) {
+            const uint32_t r = r0 + lane;
+            float dd = 0.0f;
+            if (r < nr) dd = tile_row_dist<MT, PREC, !TC>(stage + (size_t)r * ly.sstride, qf, sc, a.lp_chunks);
+            const bool keep = r < nr && dd < cutoff;
+            const unsigned m = __ballot_sync(FULL, keep);
+            uint32_t at = 0;
+            if (lane == 0 && m) at = atomicAdd(misc + 2, (uint32_t)__popc(m));
+            at = __shfl_sync(FULL, at, 0);
+            if (keep) cand[at + __popc(m & ((1u << lane) - 1u))] = make_key(dd, cid[c0 + r]);
           }
         }
         __syncthreads();  // the next round overwrites the staged rows (and the accumulator)
@@ -412,23 +448,30 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
       cmps += ncand;
       const uint32_t nc = misc[2];
       if (nc > 0) {
-        // ---- merge by rank: keys are distinct (ids are), visited flags ignored in the order
-        for (uint32_t i = tid; i < fn; i += blockDim.x) {
-          const uint64_t key = fr[i], mk = key & PANN_KEYMASK;
-          uint32_t r = i;
-          for (uint32_t j = 0; j < nc; j++) r += cand[j] < mk;
-          if (r < L) fr2[r] = key;
-        }
-        for (uint32_t j = tid; j < nc; j += blockDim.x) {
-          const uint64_t ck = cand[j];
-          uint32_t lo = 0, hi = fn;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if ((fr[mid] & PANN_KEYMASK) < ck) lo = mid + 1; else hi = mid;
+        // ---- merge by rank: keys are distinct (ids are), visited flags ignored in the order; the first half of
+        // the threads places the frontier's entries, the other half the candidates
+        const uint32_t ht = blockDim.x / 2;
+        if ((uint32_t)tid < ht) {
+          for (uint32_t i = tid; i < fn; i += ht) {
+            const uint64_t key = fr[i], mk = key & PANN_KEYMASK;
+            uint32_t r = i;
+#pragma unroll 4
+            for (uint32_t j = 0; j < nc; j++) r += cand[j] < mk;
+            if (r < L) fr2[r] = key;
           }
-          uint32_t r = lo;
-          for (uint32_t t = 0; t < nc; t++) r += cand[t] < ck;
-          if (r < L) fr2[r] = ck;
+        } else {
+          for (uint32_t j = tid - ht; j < nc; j += ht) {
+            const uint64_t ck = cand[j];
+            uint32_t lo = 0, hi = fn;
+            while (lo < hi) {
+              const uint32_t mid = (lo + hi) >> 1;
+              if ((fr[mid] & PANN_KEYMASK) < ck) lo = mid + 1; else hi = mid;
+            }
+            uint32_t r = lo;
+#pragma unroll 4
+            for (uint32_t t = 0; t < nc; t++) r += cand[t] < ck;
+            if (r < L) fr2[r] = ck;
+          }
         }
         fn = fn + nc < L ? fn + nc : L;
         uint64_t* t = fr; fr = fr2; fr2 = t;
@@ -439,10 +482,31 @@ __global__ void __launch_bounds__(128) search_tile_kernel(SearchArgs a, uint32_t
     // ---- exact float32 re-rank of the best entries, then the top k
     const uint32_t rr = a.rerank ? a.rerank : 4 * kq;
     const uint32_t nr = fn < (rr > kq ? rr : kq) ? fn : (rr > kq ? rr : kq);
-    for (uint32_t i = tid; i < nr; i += blockDim.x) {
-      const uint32_t id = key_id(fr[i]);
-      const float dd = exact_f32_dist<MT>(reinterpret_cast<const float*>(a.points + (uint64_t)id * a.stride), qf, a.d);
-      cand[i] = make_key(dd, id);
+    {
+      // the seen table and the stage are free now: the query as the exact kernels stage it, then row buffers for as
+      // many warps as fit (rowscore.cuh); without one, a row per thread
+      uint8_t* const qs = smem + ly.table;
+      const uint32_t qb = (uint32_t)((a.stride + 15) & ~15ull);
+      const uint32_t room = (uint32_t)((TC ? ly.qb : ly.misc) - ly.table);
+      const uint32_t nwarp = room > qb ? min(4u, (room - qb) / row_score_scratch<DT_F32>()) : 0u;
+      for (uint32_t i = tid; i < (uint32_t)a.stride / 4; i += blockDim.x) {
+        const float x = i < a.d ? qf[i] : 0.0f;
+        reinterpret_cast<float*>(qs)[i] = MT == MT_L2 ? -x : x;
+      }
+      __syncthreads();
+      if (nwarp > 0) {
+        for (uint32_t b = 32 * warp; (uint32_t)warp < nwarp && b < nr; b += 32 * nwarp) {
+          const uint32_t id = b + lane < nr ? key_id(fr[b + lane]) : 0u;
+          const float dd = warp_score_rows<DT_F32, MT>(a.points, a.stride, (int)a.nchunks, id, (int)min(32u, nr - b),
+                                                       qs, qs + qb + warp * row_score_scratch<DT_F32>(), 0, lane);
+          if (b + lane < nr) cand[b + lane] = make_key(dd, id);
+        }
+      } else {
+        for (uint32_t i = tid; i < nr; i += blockDim.x) {
+          const uint32_t id = key_id(fr[i]);
+          cand[i] = make_key(point_dist<DT_F32, MT>(a.points + (uint64_t)id * a.stride, qs, (int)a.d, (int)a.nchunks, 0), id);
+        }
+      }
     }
     __syncthreads();
     uint32_t* const oid = a.out_ids + (uint64_t)qi * a.kstride;
