@@ -256,19 +256,21 @@ cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const Search
   return cudaErrorInvalidValue;
 }
 
-template <int DT, int MT>
+template <int DT, int MT, bool SM>
 static cudaError_t launch_emulate_block_t(const SearchArgs& a, const EmuArgs& e, int blocks, size_t smem,
                                           cudaStream_t st) {
-  auto k = search_emulate_block_kernel<DT, MT, EMU_BLOCK_WARPS, 24>;
+  auto k = search_emulate_block_kernel<DT, MT, EMU_BLOCK_WARPS, 24, SM>;
   cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
   if (err != cudaSuccess) return err;
   k<<<blocks, 32 * EMU_BLOCK_WARPS, smem, st>>>(a, e);
   return cudaGetLastError();
 }
-cudaError_t launch_emulate_block(int dtype, int metric, const SearchArgs& a, const EmuArgs& e, int blocks, size_t smem,
-                                 cudaStream_t st) {
-#define PANN_EMUB_CASE(DT, MT) \
-  if (dtype == DT && metric == MT) return launch_emulate_block_t<DT, MT>(a, e, blocks, smem, st);
+cudaError_t launch_emulate_block(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
+                                 int blocks, size_t smem, cudaStream_t st) {
+#define PANN_EMUB_CASE(DT, MT)                                                                   \
+  if (dtype == DT && metric == MT)                                                               \
+    return smem_tables ? launch_emulate_block_t<DT, MT, true>(a, e, blocks, smem, st)            \
+                       : launch_emulate_block_t<DT, MT, false>(a, e, blocks, smem, st);
   PANN_EMUB_CASE(DT_U8, MT_L2)
   PANN_EMUB_CASE(DT_U8, MT_IP)
   PANN_EMUB_CASE(DT_I8, MT_L2)
@@ -277,6 +279,17 @@ cudaError_t launch_emulate_block(int dtype, int metric, const SearchArgs& a, con
   PANN_EMUB_CASE(DT_F32, MT_IP)
 #undef PANN_EMUB_CASE
   return cudaErrorInvalidValue;
+}
+
+// The emulation with its tables in global memory: a block per query where the
+// block's state fits in shared memory, else a warp.
+static cudaError_t launch_emulate_global(const pann_index* idx, const SearchPlan& plan, const TierSizes& z,
+                                         const SearchArgs& a, const EmuArgs& e, cudaStream_t st) {
+  const size_t smem = emu_block_layout(idx->stride, plan.L, plan.Ccap, idx->R, z.vs, 0, 0).bytes;
+  const int blocks = (int)std::min<uint64_t>(z.e2_slots, std::max<uint32_t>(a.nq, 1));
+  if (smem <= idx->smem_optin)
+    return launch_emulate_block(idx->dtype, idx->metric, false, a, e, blocks, smem, st);
+  return launch_emulate(idx->dtype, idx->metric, false, a, e, z.e2_slots, emu_smem_bytes(z.base, z.vs, 0, 0, false), st);
 }
 
 template <int DT, int MT, int SEEN, int PREC = PREC_F32>
@@ -519,7 +532,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
       e.overflow_rec = b.ovf_rec;
       e.overflow_count = cnt + 8;
       e.job_rec = nullptr;
-      PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, c, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
+      PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, true, c, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
                                      z.emu_smem_need, st));
       EmuArgs e2 = e;
       e2.gA = b.ge2;
@@ -533,8 +546,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
       c.job_list = b.ovf;
       c.njobs_dev = cnt + 8;
       c.job_counter = cnt + 7;
-      PANN_CUDA(launch_emulate(idx->dtype, idx->metric, false, c, e2, z.e2_slots,
-                               emu_smem_bytes(z.base, z.vs, 0, 0, false), st));
+      PANN_CUDA(launch_emulate_global(idx, plan, z, c, e2, st));
       return PANN_OK;
     }
     if (phase & TIERS_FIRST)
@@ -562,7 +574,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
     e.overflow_count = cnt + 8;
     e.job_rec = b.emu_rec;
     e.early = 1;
-    PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, t, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
+    PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, true, t, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
                                    z.emu_smem_need, side));
     PANN_CUDA(cudaEventRecord(idx->ev_join, side));
   }
@@ -610,7 +622,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
       t.job_counter = cnt + 5;
       // no more blocks than queries: each needs most of an SM's shared memory,
       // so a small search beside other work on the device asks for few SMs
-      PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, t, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
+      PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, true, t, e, (int)std::min<uint64_t>(idx->sm_count, a.nq),
                                      z.emu_smem_need, st));
       glist = b.ovf;
       grec = b.ovf_rec;
@@ -629,8 +641,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
     t.job_list = glist;
     t.njobs_dev = gcount;
     t.job_counter = cnt + 7;
-    PANN_CUDA(launch_emulate(idx->dtype, idx->metric, false, t, e, z.e2_slots, emu_smem_bytes(z.base, z.vs, 0, 0, false),
-                             st));
+    PANN_CUDA(launch_emulate_global(idx, plan, z, t, e, st));
   }
   return PANN_OK;
 }

@@ -980,8 +980,9 @@ __global__ void __launch_bounds__(32) search_emulate_kernel(SearchArgs a, EmuArg
 }
 
 // ---------------------------------------------------------------------------
-// The same emulation with one block of NW warps per query (shared-memory
-// tables only). The per-visit work that does not touch the reference's table
+// The same emulation with one block of NW warps per query, its tables in shared
+// memory (SMEM) or, for beams whose tables do not fit there, in global memory
+// per resident block. The per-visit work that does not touch the reference's table
 // runs beside it: warp 0 makes the hashset calls in order, while warps
 // 1..NW-1 score every neighbour of the visited node (each thread one whole
 // row, all its loads in flight at once), so the rows arrive while the table
@@ -1084,13 +1085,14 @@ __device__ __forceinline__ int block_merge(const uint64_t* fr, int fn, const uin
   return t < L ? t : L;
 }
 
-template <int DT, int MT, int NW, int CH>
+template <int DT, int MT, int NW, int CH, bool SMEM>
 __global__ void __launch_bounds__(NW * 32, 1) search_emulate_block_kernel(SearchArgs a, EmuArgs e) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nth = NW * 32;
   const unsigned FULL = 0xFFFFFFFFu;
-  const EmuBlockLayout y = emu_block_layout(a.stride, a.L, a.Ccap, a.R, e.vs_slots, e.capA, e.capB);
+  const EmuBlockLayout y =
+      emu_block_layout(a.stride, a.L, a.Ccap, a.R, e.vs_slots, SMEM ? e.capA : 0, SMEM ? e.capB : 0);
   uint8_t* qs = smem;
   uint64_t* frA = reinterpret_cast<uint64_t*>(smem + y.fr);
   uint64_t* frB = frA + a.L;
@@ -1101,8 +1103,8 @@ __global__ void __launch_bounds__(NW * 32, 1) search_emulate_block_kernel(Search
   float* dall = reinterpret_cast<float*>(smem + y.dall);
   volatile uint32_t* ctrl = reinterpret_cast<volatile uint32_t*>(smem + y.ctrl);
   uint32_t* vset = reinterpret_cast<uint32_t*>(smem + y.vset);
-  uint32_t* tabA = reinterpret_cast<uint32_t*>(smem + y.tabA);
-  uint32_t* tabB = reinterpret_cast<uint32_t*>(smem + y.tabB);
+  uint32_t* const tabA = SMEM ? reinterpret_cast<uint32_t*>(smem + y.tabA) : e.gA + (size_t)blockIdx.x * e.capA;
+  uint32_t* const tabB = SMEM ? reinterpret_cast<uint32_t*>(smem + y.tabB) : e.gB + (size_t)blockIdx.x * e.capB;
   const uint32_t vmask = e.vs_slots - 1;
   const uint32_t nel = a.dl < a.R ? a.dl : a.R;
 

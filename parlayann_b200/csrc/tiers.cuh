@@ -52,10 +52,10 @@ cudaError_t launch_search(int dtype, int metric, int seen, const SearchArgs& a, 
                           size_t smem, cudaStream_t st, int prec, int minb = 3);
 cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
                            int blocks, size_t smem, cudaStream_t st);
-// Warps per block of the shared-memory emulation tier (one query per block).
+// Warps per block of the block-per-query emulation.
 constexpr int EMU_BLOCK_WARPS = 4;
-cudaError_t launch_emulate_block(int dtype, int metric, const SearchArgs& a, const EmuArgs& e, int blocks, size_t smem,
-                                 cudaStream_t st);
+cudaError_t launch_emulate_block(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
+                                 int blocks, size_t smem, cudaStream_t st);
 // Tier 0's table, warps and blocks (S_force, wpb_force: 0 = automatic).
 int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
                 int wpb_force, int minb, TierSizes* z);
