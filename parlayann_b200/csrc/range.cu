@@ -9,7 +9,7 @@
 //      entries within the radius are a prefix. A Greedy query whose whole
 //      frontier is in range becomes an expansion job; every other query's
 //      answer is that prefix.
-//   3. range_expand_kernel: greedy_search (rangeSearch.h:21-55), one warp per
+//   3. range_expand_kernel: greedy_search (rangeSearch.h:21-55), one block per
 //      query. Its FIFO order is the answer's order and its hashset
 //      (hashset.h:13-55, initial capacity 2 * beam * 64) decides which
 //      neighbours count as new, so the warp runs the reference's sequence of
@@ -31,12 +31,13 @@
 
 #include "common.cuh"
 #include "index.cuh"
+#include "rowscore.cuh"
 #include "tiers.cuh"
 
 namespace pann {
 
 enum RangeStatus : uint32_t { RS_RETRY = 1u, RS_GREW = 2u };
-constexpr int HOME_BATCH = 8;      // table loads in flight per thread
+constexpr int GATHER_BATCH = 8;    // adjacency entries and table slots in flight per thread
 constexpr int EXPAND_THREADS = 256;  // one block per expansion
 
 struct RangeArgs {
@@ -143,26 +144,41 @@ __device__ __forceinline__ uint32_t block_compact(const uint32_t* tmp, uint32_t 
 // Block control words in shared memory; CTL_CUR (the table pointer) and
 // CTL_OFF (the answer pool offset) are 64-bit, at 8-byte aligned words.
 enum : uint32_t {
-  CTL_JOB = 0, CTL_OK, CTL_COUNT, CTL_NUN, CTL_FILTERED = 5, CTL_BITS, CTL_TOT, CTL_CUR = 8, CTL_OFF = 10, CTL_WORDS = 16
+  CTL_JOB = 0, CTL_OK, CTL_COUNT, CTL_NUN, CTL_FILTERED = 5, CTL_BITS, CTL_TOT, CTL_CUR = 8, CTL_OFF = 10,
+  CTL_GROW = 12, CTL_SIDE, CTL_OTHER_CAP, CTL_GROW_SCRATCH = 16, CTL_WORDS = 32
 };
 
 // One block per query (EXPAND_THREADS threads). Warp 0 owns the emulated
 // hashset and makes its calls in order; every warp gathers adjacency rows,
 // looks keys up in the table as it stands, scores new neighbours and takes
 // part in the ordered compactions.
+//
+// Bounded by the latency of the longest expansion: a round of 32 nodes passes
+// eight block barriers and five dependent trips to L2, with two blocks an SM.
+// So a round keeps as much in flight as it can: rows, then table slots, eight
+// a thread, without a barrier between them; one pass that places the calls;
+// rows scored 32 a warp (warp_score_rows); a growth on the whole block. 193
+// expansions of ~3,900 answers (200K x 96 float, R 64): 3.4 -> 1.5 ms. A
+// round spent 5.6K of its 36K cycles on warp 0 counting the calls, 6K on
+// gathering, 3.4K each on compacting and looking up, 8.5K on the calls and,
+// averaged, 4.5K on growths.
 template <int DT, int MT>
-__global__ void __launch_bounds__(EXPAND_THREADS) range_expand_kernel(RangeArgs a) {
+__global__ void __launch_bounds__(EXPAND_THREADS, 2) range_expand_kernel(RangeArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const unsigned FULL = 0xFFFFFFFFu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t nthr = blockDim.x;
   const unsigned lt = (1u << lane) - 1u;
   uint8_t* qs = smem;
-  uint32_t* kbuf = reinterpret_cast<uint32_t*>(smem + a.stride);
+  uint32_t* kbuf = reinterpret_cast<uint32_t*>(smem + a.stride + (EXPAND_THREADS / 32 - 1) * row_score_scratch<DT>());
   uint32_t* ubuf = kbuf + a.keybuf;
   uint32_t* kraw = ubuf + a.keybuf;  // a round's adjacency rows as loaded
+  // scoring scratch: kraw (8 KB or more) holds nothing while a round's new neighbours are scored
+  uint8_t* stg = warp == 0 ? reinterpret_cast<uint8_t*>(kraw) : smem + a.stride + (warp - 1) * row_score_scratch<DT>();
   uint32_t* ctl = kraw + a.keybuf;
   uint32_t* ccnt = ctl + CTL_WORDS;
+  uint32_t* mlive = ccnt + a.keybuf / 32 + 2;  // per 32 gathered entries: live ones, ones not in the table
+  uint32_t* mmiss = mlive + a.keybuf / 32 + 2;
   uint32_t* tabA = a.tabs + (size_t)blockIdx.x * 2 * a.cap;
   uint32_t* tabB = tabA + a.cap;
   uint32_t* Q = a.queues + (size_t)blockIdx.x * a.qcap;
@@ -215,25 +231,19 @@ __global__ void __launch_bounds__(EXPAND_THREADS) range_expand_kernel(RangeArgs 
     uint32_t count = ctl[CTL_COUNT];
 
     // breadth-first expansion (rangeSearch.h:36-52), up to gn queued nodes a
-    // round: their adjacency rows are gathered together (one memory round
-    // trip), the hash homes of all their neighbours and the next round's rows
-    // are prefetched into L2, the hashset calls run in order, and the rows of
-    // the new neighbours are prefetched as the calls find them
-    const uint32_t gn = a.keybuf / a.R > 0 ? a.keybuf / a.R : 1;
+    // round: their adjacency rows are gathered and looked up together, the
+    // next round's rows are prefetched into L2, the hashset calls run in order,
+    // and the rows of the new neighbours are prefetched as the calls find them
+    const uint32_t rc = (a.R + 31) / 32, nw = nthr / 32;  // 32-entry parts of a row
+    const uint32_t gn = a.keybuf / (32 * rc);
     const uint32_t row_lines = (a.R * 4 + 127) / 128;
     uint32_t pos = 0;
     while (ok && pos < count) {
       const uint32_t end = count - pos < gn ? count : pos + gn;
-      const uint32_t nraw = (end - pos) * a.R;
+      const uint32_t nch = (end - pos) * rc;
       const uint32_t bits = ctl[CTL_BITS];
       const uint32_t* tab = *reinterpret_cast<uint32_t* const*>(ctl + CTL_CUR);
       const uint32_t mask0 = (1u << bits) - 1u;
-      for (uint32_t i = tid; i < nraw; i += nthr) {
-        const uint32_t node = Q[pos + i / a.R];
-        const uint32_t v = __ldg(a.graph + (uint64_t)node * a.R + (i % a.R));
-        kraw[i] = v;
-        if (v != PANN_PAD) asm volatile("prefetch.global.L2 [%0];" ::"l"(tab + ref_slot(v, mask0)));
-      }
       {  // the next round's rows (nodes queued so far)
         const uint32_t nend = count - end < gn ? count : end + gn;
         for (uint32_t i = tid; i < (nend - end) * row_lines; i += nthr) {
@@ -241,10 +251,9 @@ __global__ void __launch_bounds__(EXPAND_THREADS) range_expand_kernel(RangeArgs 
           asm volatile("prefetch.global.L2 [%0];" ::"l"(a.graph + (uint64_t)node * a.R + 32 * (i % row_lines)));
         }
       }
-      __syncthreads();
-      // the neighbours in order (a row's live entries are those before PAD)
-      const uint32_t nk = block_compact(kraw, nraw, kbuf, a.keybuf, ccnt, ctl + CTL_TOT);
-      // A call whose key the table already holds on its probe path (its home
+      // A warp takes 32 entries of a row at a time (a row's live entries are
+      // those before PAD), GATHER_BATCH of them in flight, and looks their keys
+      // up. A call whose key the table already holds on its probe path (its home
       // slot, then the slots after it up to the first empty one) returns true
       // and changes nothing (hashset.h:22-24,39-44) unless the table grows
       // first (hashset.h:25). Slots are only ever emptied by a growth, and the
@@ -252,74 +261,184 @@ __global__ void __launch_bounds__(EXPAND_THREADS) range_expand_kernel(RangeArgs 
       // So the round's calls are looked up against the table as it stands;
       // when even every call not found there inserting keeps num_entries at
       // or below half, only those calls run, in order; otherwise all of them.
-      for (uint32_t b0 = 0; b0 < nk; b0 += nthr * HOME_BATCH) {
-        uint32_t hv[HOME_BATCH];
+      uint32_t nd = warp / rc, part = warp % rc;
+      for (uint32_t c0 = 0; c0 < nch; c0 += nw * GATHER_BATCH) {
+        uint32_t node[GATHER_BATCH], off[GATHER_BATCH], v[GATHER_BATCH], hv[GATHER_BATCH];
 #pragma unroll
-        for (int j = 0; j < HOME_BATCH; j++) {
-          const uint32_t i = b0 + nthr * j + tid;
-          hv[j] = i < nk ? tab[ref_slot(kbuf[i], mask0)] : PANN_PAD;
+        for (int j = 0; j < GATHER_BATCH; j++) {
+          off[j] = part * 32 + lane;
+          if (c0 + nw * j + warp >= nch) off[j] = a.R;
+          node[j] = off[j] < a.R ? Q[pos + nd] : 0u;
+          nd += nw / rc;
+          part += nw % rc;
+          if (part >= rc) { part -= rc; nd++; }
         }
 #pragma unroll
-        for (int j = 0; j < HOME_BATCH; j++) {
-          const uint32_t i = b0 + nthr * j + tid;
-          if (i < nk) {
-            const uint32_t key = kbuf[i];
-            uint32_t v = hv[j];
-            uint32_t p = ref_slot(key, mask0);
-            for (uint32_t s = 0; v != PANN_PAD && v != key && s < mask0; s++) {
+        for (int j = 0; j < GATHER_BATCH; j++)
+          v[j] = off[j] < a.R ? __ldg(a.graph + (uint64_t)node[j] * a.R + off[j]) : PANN_PAD;
+#pragma unroll
+        for (int j = 0; j < GATHER_BATCH; j++) hv[j] = v[j] != PANN_PAD ? tab[ref_slot(v[j], mask0)] : PANN_PAD;
+#pragma unroll
+        for (int j = 0; j < GATHER_BATCH; j++) {
+          const uint32_t c = c0 + nw * j + warp;
+          if (c < nch) {
+            const uint32_t key = v[j];
+            uint32_t t = hv[j], p = ref_slot(key, mask0);
+            for (uint32_t s = 0; t != PANN_PAD && t != key && s < mask0; s++) {
               p = (p + 1) & mask0;
-              v = tab[p];
+              t = tab[p];
             }
-            kraw[i] = v == key ? PANN_PAD : key;
+            const unsigned live = __ballot_sync(FULL, key != PANN_PAD);
+            const unsigned miss = __ballot_sync(FULL, key != PANN_PAD && t != key);
+            kraw[c * 32 + lane] = key;
+            if (lane == 0) {
+              mlive[c] = live;
+              mmiss[c] = miss;
+            }
           }
         }
       }
       __syncthreads();
-      // warp 0 decides; the kept calls replace kbuf only on the fast path
+      // warp 0 decides which calls run and where each chunk's go
       if (warp == 0) {
         uint32_t nf = 0;
-        for (uint32_t c0 = 0; c0 < nk; c0 += 32)
-          nf += __popc(__ballot_sync(FULL, c0 + lane < nk && kraw[c0 + lane] != PANN_PAD));
-        if (lane == 0) ctl[CTL_FILTERED] = h.num_entries + (long long)nf <= (long long)((1u << h.bits) / 2);
-      }
-      __syncthreads();
-      uint32_t ncalls = nk;
-      if (ctl[CTL_FILTERED]) ncalls = block_compact(kraw, nk, kbuf, a.keybuf, ccnt, ctl + CTL_TOT);
-      // the hashset calls, in order (warp 0)
-      if (warp == 0) {
-        uint32_t nun = 0;
-        bool wok = true;
-        for (uint32_t k0 = 0; k0 < ncalls && wok; k0 += 32) {
-          const bool valid = k0 + lane < ncalls;
-          const uint32_t key = valid ? kbuf[k0 + lane] : PANN_PAD;
-          bool seen = false;
-          wok = emu_batch(h, key, valid, lane, &seen);
-          const bool un = wok && valid && !seen;
-          const unsigned m = __ballot_sync(FULL, un);
-          if (un) {
-            ubuf[nun + __popc(m & lt)] = key;
-            const char* row = reinterpret_cast<const char*>(a.points + (uint64_t)key * a.stride);
-            for (uint32_t o = 0; o < a.stride; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + o));
+        for (uint32_t c = lane; c < nch; c += 32) nf += __popc(mmiss[c]);
+        nf = __reduce_add_sync(FULL, nf);
+        const bool filtered = h.num_entries + (long long)nf <= (long long)((1u << h.bits) / 2);
+        uint32_t carry = 0;
+        for (uint32_t c0 = 0; c0 < nch; c0 += 32) {
+          const uint32_t m = c0 + lane < nch ? (filtered ? mmiss[c0 + lane] : mlive[c0 + lane]) : 0u;
+          const uint32_t n = __popc(m);
+          uint32_t incl = n;
+#pragma unroll
+          for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, incl, s);
+            if (lane >= s) incl += t;
           }
-          nun += __popc(m);
+          if (c0 + lane < nch) {
+            mlive[c0 + lane] = m;
+            ccnt[c0 + lane] = carry + incl - n;
+          }
+          carry += __shfl_sync(FULL, incl, 31);
         }
         if (lane == 0) {
-          ctl[CTL_OK] = wok;
-          ctl[CTL_NUN] = nun;
-          ctl[CTL_BITS] = h.bits;
-          *reinterpret_cast<uint32_t**>(ctl + CTL_CUR) = h.cur;
+          ctl[CTL_FILTERED] = filtered;
+          ctl[CTL_TOT] = carry;
         }
       }
       __syncthreads();
+      const uint32_t ncalls = ctl[CTL_TOT];
+      const bool filtered = ctl[CTL_FILTERED] != 0;
+      for (uint32_t c = warp; c < nch; c += nw) {
+        const uint32_t m = mlive[c];
+        if ((m >> lane) & 1u) kbuf[ccnt[c] + __popc(m & lt)] = kraw[c * 32 + lane];
+      }
+      __syncthreads();
+      // the hashset calls, in order (warp 0). Those of a filtered round are first sight or a repeat within the round,
+      // and none can grow the table. In other rounds a call that grows the table stops them; the whole block grows it
+      // (re-inserting thousands of keys on one warp took a third of an expansion's time) and they go on after it
+      if (filtered) {
+        if (warp == 0) {
+          uint32_t nun = 0;
+          const uint32_t mask = (1u << h.bits) - 1u;
+          for (uint32_t k0 = 0; k0 < ncalls; k0 += 32) {
+            const uint32_t key = k0 + lane < ncalls ? kbuf[k0 + lane] : PANN_PAD;
+            bool ins;
+            uint32_t at;
+            emu_probe_rounds(h.cur, mask, key, key != PANN_PAD, ref_slot(key, mask), lane, &ins, &at);
+            const unsigned m = __ballot_sync(FULL, ins);
+            if (ins) {
+              ubuf[nun + __popc(m & lt)] = key;
+              const char* row = reinterpret_cast<const char*>(a.points + (uint64_t)key * a.stride);
+              for (uint32_t o = 0; o < a.stride; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + o));
+            }
+            nun += __popc(m);
+          }
+          h.num_entries += nun;
+          if (lane == 0) ctl[CTL_NUN] = nun;
+        }
+        __syncthreads();
+      } else {
+        uint32_t nun = 0, k0 = 0, key = PANN_PAD;  // warp 0's state
+        unsigned pend = 0;
+        bool wok = true, open = false, seen = false;
+        int g = -1;
+        for (;;) {
+          if (warp == 0) {
+            g = -1;
+            while (wok) {
+              if (!open) {
+                if (k0 >= ncalls) break;
+                key = k0 + lane < ncalls ? kbuf[k0 + lane] : PANN_PAD;
+                pend = __ballot_sync(FULL, key != PANN_PAD);
+                seen = false;
+                open = true;
+              }
+              if (pend) {
+                emu_batch_part(h, key, (pend >> lane) & 1u, lane, &seen, &g);
+                if (g >= 0) {
+                  pend &= ~((2u << g) - 1u);
+                  break;
+                }
+                pend = 0;
+              }
+              const bool un = key != PANN_PAD && !seen;
+              const unsigned m = __ballot_sync(FULL, un);
+              if (un) {
+                ubuf[nun + __popc(m & lt)] = key;
+                const char* row = reinterpret_cast<const char*>(a.points + (uint64_t)key * a.stride);
+                for (uint32_t o = 0; o < a.stride; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + o));
+              }
+              nun += __popc(m);
+              k0 += 32;
+              open = false;
+            }
+            const uint32_t gkey = __shfl_sync(FULL, key, g < 0 ? 0 : g);
+            if (lane == 0) {
+              ctl[CTL_GROW] = g >= 0 ? gkey : PANN_PAD;
+              ctl[CTL_SIDE] = h.cur == tabB;
+              ctl[CTL_BITS] = h.bits;
+              ctl[CTL_OTHER_CAP] = h.other_cap;
+              ctl[CTL_OK] = wok;
+              ctl[CTL_NUN] = nun;
+              *reinterpret_cast<uint32_t**>(ctl + CTL_CUR) = h.cur;
+            }
+          }
+          __syncthreads();
+          const uint32_t gk = ctl[CTL_GROW];
+          if (gk == PANN_PAD) break;
+          uint32_t* const gcur = ctl[CTL_SIDE] ? tabB : tabA;
+          uint32_t* const goth = ctl[CTL_SIDE] ? tabA : tabB;
+          uint32_t added = 0;
+          bool aseen = false;
+          const bool grew = emu_grow_block(gcur, goth, ctl[CTL_BITS], ctl[CTL_OTHER_CAP], gk, tid, (int)nthr,
+                                           ctl + CTL_GROW_SCRATCH, &added, &aseen);
+          if (warp == 0) {
+            if (!grew) {
+              wok = false;
+            } else {
+              h.num_entries += added;
+              uint32_t* t = h.cur; h.cur = h.other; h.other = t;
+              const uint32_t c = h.cur_cap; h.cur_cap = h.other_cap; h.other_cap = c;
+              h.bits += 1;
+              if (!aseen) h.num_entries++;
+              if (lane == g) seen = aseen;
+            }
+          }
+          __syncthreads();
+        }
+      }
       ok = ctl[CTL_OK] != 0;
       if (!ok) break;
       const uint32_t nun = ctl[CTL_NUN];
       cmps += nun;
-      // distances of the new neighbours; in-range ones join the queue in order
-      for (uint32_t u = tid; u < nun; u += nthr) {
-        const uint32_t id = ubuf[u];
-        const float dd = point_dist<DT, MT>(a.points + (uint64_t)id * a.stride, qs, (int)a.d, (int)a.nchunks, qq);
-        kbuf[u] = (double)dd <= a.radius ? id : PANN_PAD;
+      // distances of the new neighbours, 32 a warp; in-range ones join the queue in order
+      for (uint32_t u0 = 32 * warp; u0 < nun; u0 += nthr) {
+        const uint32_t u = u0 + lane;
+        const uint32_t id = u < nun ? ubuf[u] : 0u;
+        const float dd = warp_score_rows<DT, MT>(a.points, a.stride, (int)a.nchunks, id, (int)min(32u, nun - u0), qs, stg,
+                                                 qq, lane);
+        if (u < nun) kbuf[u] = (double)dd <= a.radius ? id : PANN_PAD;
       }
       __syncthreads();
       count += block_compact(kbuf, nun, Q + count, a.qcap - count, ccnt, ctl + CTL_TOT);
@@ -517,7 +636,8 @@ extern "C" int pann_range_search(pann_index* idx, const void* queries, uint32_t 
     cap0 = std::max(cap0, bits0 + 2);
     const Tier tiers[2] = {{cap0, cap0 - 2, 2 * idx->sm_count}, {std::max<uint32_t>(24, bits0 + 2), 22, 16}};
     const uint32_t keybuf = (std::max<uint32_t>(2048, idx->R) + 31) & ~31u;  // 8-byte aligned control words
-    const size_t smem = idx->stride + 12ull * keybuf + 4ull * (CTL_WORDS + keybuf / 32 + 2);
+    const size_t smem = idx->stride + (EXPAND_THREADS / 32 - 1) * (size_t)row_score_scratch_rt(idx->dtype) +
+                        12ull * keybuf + 4ull * (CTL_WORDS + 3 * (keybuf / 32 + 2));
     unsigned long long pool_cap = std::max<unsigned long long>(1ull << 22, 256ull * h_njobs);
     for (int attempt = 0; attempt < 3; attempt++) {
       PANN_CUDA(idx->range_pool.ensure_grow(4 * pool_cap));

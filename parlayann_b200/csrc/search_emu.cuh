@@ -494,26 +494,45 @@ __device__ __forceinline__ void emu_batch_part(EmuHash& h, uint32_t key, bool ac
 // 8 keys replayed by their owner thread, longer ones by one warp each;
 // beyond EMU_LONG_CLUSTER keys, or more long clusters than the free tail
 // lists, a sequential pass by thread 0. ctl: 4 words of shared scratch.
+// What bounds it is the latency of the tables' loads (L2 when they lie in
+// global memory), so each pass keeps four ranks or sixteen slots a thread in
+// flight; one at a time, the growth of a 16K-slot table took 280K cycles.
 __device__ __forceinline__ void emu_place_ranked_block(uint32_t* keys, uint32_t cnt, uint32_t* other, uint32_t nmask,
                                                        uint32_t tail_words, int tid, int nth, volatile uint32_t* ctl) {
   const unsigned FULL = 0xFFFFFFFFu;
   const int lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
   const uint32_t nsize = nmask + 1;
   volatile uint32_t* vo = other;
-  for (uint32_t r = (uint32_t)tid; r < cnt; r += (uint32_t)nth) {
-    const uint32_t k = keys[r];
-    uint32_t p = ref_slot(k, nmask);
-    for (;;) {
-      uint32_t w = vo[p];
-      if (w == PANN_PAD) {
-        w = atomicCAS(other + p, PANN_PAD, r);
-        if (w == PANN_PAD) break;
+  for (uint32_t r0 = (uint32_t)tid; r0 < cnt; r0 += 4u * (uint32_t)nth) {
+    uint32_t k[4], p[4], w[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t r = r0 + (uint32_t)(j * nth);
+      k[j] = r < cnt ? keys[r] : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      p[j] = ref_slot(k[j], nmask);
+      w[j] = vo[p[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t r = r0 + (uint32_t)(j * nth);
+      if (r < cnt && w[j] == PANN_PAD) w[j] = atomicCAS(other + p[j], PANN_PAD, r);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t r = r0 + (uint32_t)(j * nth);
+      uint32_t at = p[j], u = w[j];
+      while (r < cnt && u != PANN_PAD) {  // PAD: the slot was empty and is this rank's now
+        if (keys[u] == k[j]) {
+          atomicMin(other + at, r);
+          break;
+        }
+        at = (at + 1) & nmask;
+        u = vo[at];
+        if (u == PANN_PAD) u = atomicCAS(other + at, PANN_PAD, r);
       }
-      if (keys[w] == k) {
-        atomicMin(other + p, r);
-        break;
-      }
-      p = (p + 1) & nmask;
     }
   }
   const uint32_t nb = (cnt + 31) / 32;
@@ -524,19 +543,56 @@ __device__ __forceinline__ void emu_place_ranked_block(uint32_t* keys, uint32_t 
   if (tid == 0) { ctl[0] = 0; ctl[1] = 0; }
   for (uint32_t b = (uint32_t)tid; b < nb; b += (uint32_t)nth) owner[b] = 0;
   __syncthreads();
-  for (uint32_t p = (uint32_t)tid; p < nsize; p += (uint32_t)nth) {
-    const uint32_t w = vo[p];
-    if (w != PANN_PAD && vo[(p - 1) & nmask] == PANN_PAD) atomicOr(owner + (w >> 5), 1u << (w & 31));
+  for (uint32_t q0 = (uint32_t)tid; q0 < (nsize >> 2); q0 += 4u * (uint32_t)nth) {
+    uint4 x[4];
+    uint32_t pv[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t q = q0 + (uint32_t)(j * nth);
+      x[j] = make_uint4(PANN_PAD, PANN_PAD, PANN_PAD, PANN_PAD);
+      pv[j] = 0u;
+      if (q < (nsize >> 2)) {
+        x[j] = reinterpret_cast<const uint4*>(other)[q];
+        pv[j] = other[(4 * q - 1) & nmask];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t s[5] = {pv[j], x[j].x, x[j].y, x[j].z, x[j].w};
+#pragma unroll
+      for (int t = 1; t < 5; t++)
+        if (s[t] != PANN_PAD && s[t - 1] == PANN_PAD) atomicOr(owner + (s[t] >> 5), 1u << (s[t] & 31));
+    }
   }
   __syncthreads();
-  for (uint32_t r = (uint32_t)tid; r < cnt; r += (uint32_t)nth) {
-    if (!((owner[r >> 5] >> (r & 31)) & 1u)) continue;
-    const uint32_t s0 = ref_slot(keys[r], nmask);  // an owner sits at its home
-    uint32_t m = 1;
-    while (m <= 8 && vo[(s0 + m) & nmask] != PANN_PAD) m++;
-    if (m == 1) {
-      other[s0] = keys[r];
-    } else if (m <= 8) {
+  for (uint32_t r0 = (uint32_t)tid; r0 < cnt; r0 += 4u * (uint32_t)nth) {
+    uint32_t k[4], n1[4];
+    uint32_t own = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t r = r0 + (uint32_t)(j * nth);
+      k[j] = r < cnt ? keys[r] : 0u;
+      if (r < cnt) own |= ((owner[r >> 5] >> (r & 31)) & 1u) << j;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) n1[j] = vo[(ref_slot(k[j], nmask) + 1) & nmask];  // an owner sits at its home
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (((own >> j) & 1u) && n1[j] == PANN_PAD) {
+        other[ref_slot(k[j], nmask)] = k[j];
+        own &= ~(1u << j);
+      }
+    while (own) {
+      const int jo = __ffs(own) - 1;
+      own &= own - 1;
+      const uint32_t s0 = ref_slot(jo == 0 ? k[0] : jo == 1 ? k[1] : jo == 2 ? k[2] : k[3], nmask);
+      uint32_t m = 2;
+      while (m <= 8 && vo[(s0 + m) & nmask] != PANN_PAD) m++;
+      if (m > 8) {
+        const uint32_t at = atomicAdd((uint32_t*)ctl, 1u);
+        if (at < long_cap) longs[at] = s0;
+        continue;
+      }
       uint32_t ix[8], kx[8], ox[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) ix[j] = (uint32_t)j < m ? vo[(s0 + j) & nmask] : 0xFFFFFFFFu;
@@ -560,9 +616,6 @@ __device__ __forceinline__ void emu_place_ranked_block(uint32_t* keys, uint32_t 
         taken |= 1u << pos;
         other[(s0 + pos) & nmask] = key;
       }
-    } else {
-      const uint32_t at = atomicAdd((uint32_t*)ctl, 1u);
-      if (at < long_cap) longs[at] = s0;
     }
   }
   __syncthreads();
@@ -646,15 +699,17 @@ __device__ __forceinline__ bool emu_grow_block(uint32_t* cur, uint32_t* other, u
   for (uint32_t i = (uint32_t)tid; i < (nsize >> 2); i += (uint32_t)nth) reinterpret_cast<uint4*>(other)[i] = e4;
   // the old table's keys compacted to its front in slot order
   uint32_t cnt = 0;
-  for (uint32_t base = 0; base < size; base += 4u * (uint32_t)nth) {
-    uint32_t k4[4];
+  for (uint32_t base = 0; base < size; base += 8u * (uint32_t)nth) {
+    uint32_t k8[8];
     uint32_t c = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint32_t i = base + 4 * (uint32_t)tid + (uint32_t)j;
-      k4[j] = i < size ? cur[i] : PANN_PAD;
-      c += k4[j] != PANN_PAD;
+    for (int j = 0; j < 8; j += 4) {
+      const uint32_t i = base + 8 * (uint32_t)tid + (uint32_t)j;
+      const uint4 x = i < size ? *reinterpret_cast<const uint4*>(cur + i) : e4;
+      k8[j] = x.x; k8[j + 1] = x.y; k8[j + 2] = x.z; k8[j + 3] = x.w;
     }
+#pragma unroll
+    for (int j = 0; j < 8; j++) c += k8[j] != PANN_PAD;
     uint32_t pre = c;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -672,8 +727,8 @@ __device__ __forceinline__ bool emu_grow_block(uint32_t* cur, uint32_t* other, u
     __syncthreads();
     uint32_t at = cnt + woff + pre - c;
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (k4[j] != PANN_PAD) cur[at++] = k4[j];
+    for (int j = 0; j < 8; j++)
+      if (k8[j] != PANN_PAD) cur[at++] = k8[j];
     cnt += total;
     __syncthreads();
   }
@@ -1085,6 +1140,10 @@ __device__ __forceinline__ int block_merge(const uint64_t* fr, int fn, const uin
   return t < L ? t : L;
 }
 
+// SMEM: both tables in shared memory, else in global memory (slot blockIdx.x
+// of gA and gB), where a visit waits for L2 instead; four warps that score
+// and a block that rebuilds a growing table make up for it (0.46 ms where a
+// warp per query took 1.44 ms: batch of 4,000, beams to 400, 200K x 96 float).
 template <int DT, int MT, int NW, int CH, bool SMEM>
 __global__ void __launch_bounds__(NW * 32, 1) search_emulate_block_kernel(SearchArgs a, EmuArgs e) {
   extern __shared__ __align__(16) uint8_t smem[];

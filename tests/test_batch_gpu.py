@@ -211,3 +211,22 @@ def test_batch_cta_per_query_refused_when_tables_do_not_fit(lib_built):
         idx.batch(10, 10, 200, cta_per_query=True)
     assert "CTA per query" in str(e.value)
     idx.close()
+
+
+# beams whose emulated tables lie in global memory (a block per query), on queries whose hashset grows
+@pytest.mark.parametrize("dtype,d", [(np.uint8, 8), (np.float32, 24)], ids=["u8", "f32"])
+@pytest.mark.parametrize("beam", [200, 240])
+def test_growth_with_tables_in_global_memory(dtype, d, beam, lib_built):
+    n, R = 60000, 64
+    base = random_points(dtype, n, d, 5)
+    g = O.random_graph(n, R, 6, min_deg=60)
+    q = random_points(dtype, 24, d, 7)
+    idx = P.Index(base, R)
+    idx.set_graph(g)
+    o = O.search("oracle", base, q, g, 10, beam)
+    assert (o["hash_grew"] > 0).any()
+    check(idx.search(q, 10, beam), o)
+    b = idx.batch(len(q), 10, beam)
+    check(b.run(q, 10, beam), o, "batch")
+    b.close()
+    idx.close()

@@ -199,3 +199,20 @@ def test_range_groundtruth_radius_boundary(lib_built):
     with pytest.raises(P.PannError):
         P._check(P.lib().pann_range_fetch(idx.handle, None, 0))
     idx.close()
+
+
+# rows of a part of a 32-entry chunk, just past one, and several; expansions whose table grows inside a round
+@pytest.mark.parametrize("R", [1, 5, 31, 33, 64, 100])
+@pytest.mark.parametrize("dtype,d", [(np.uint8, 10), (np.float32, 33)], ids=["u8", "f32"])
+def test_range_expansion_row_lengths(R, dtype, d, lib_built):
+    n = 20000
+    base = random_points(dtype, n, d, 91)
+    q = random_points(dtype, 12, d, 92)
+    g = O.random_graph(n, R, 93, min_deg=1)
+    idx = P.Index(base, R)
+    idx.set_graph(g)
+    for quant in (0.3, 0.9):
+        radius = sample_radius(base, q, P.L2, quant)
+        r = idx.range_search(q, 8, radius, P.RANGE_GREEDY)
+        check(r, O.range_search("oracle", base, q, g, 8, radius, O.RANGE_GREEDY), f"R={R} quant={quant}")
+    idx.close()
