@@ -283,13 +283,14 @@ cudaError_t launch_emulate_block(int dtype, int metric, bool smem_tables, const 
 
 // The emulation with its tables in global memory: a block per query where the
 // block's state fits in shared memory, else a warp.
-static cudaError_t launch_emulate_global(const pann_index* idx, const SearchPlan& plan, const TierSizes& z,
-                                         const SearchArgs& a, const EmuArgs& e, cudaStream_t st) {
-  const size_t smem = emu_block_layout(idx->stride, plan.L, plan.Ccap, idx->R, z.vs, 0, 0).bytes;
-  const int blocks = (int)std::min<uint64_t>(z.e2_slots, std::max<uint32_t>(a.nq, 1));
+cudaError_t launch_emulate_global(const pann_index* idx, const SearchPlan& plan, int slots, const SearchArgs& a,
+                                  const EmuArgs& e, cudaStream_t st) {
+  const size_t smem = emu_block_layout(idx->stride, plan.L, plan.Ccap, idx->R, e.vs_slots, 0, 0).bytes;
+  const int blocks = (int)std::min<uint64_t>(slots, std::max<uint32_t>(a.nq, 1));
   if (smem <= idx->smem_optin)
     return launch_emulate_block(idx->dtype, idx->metric, false, a, e, blocks, smem, st);
-  return launch_emulate(idx->dtype, idx->metric, false, a, e, z.e2_slots, emu_smem_bytes(z.base, z.vs, 0, 0, false), st);
+  return launch_emulate(idx->dtype, idx->metric, false, a, e, slots, emu_smem_bytes(e.base_bytes, e.vs_slots, 0, 0, false),
+                        st);
 }
 
 template <int DT, int MT, int SEEN, int PREC = PREC_F32>
@@ -546,7 +547,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
       c.job_list = b.ovf;
       c.njobs_dev = cnt + 8;
       c.job_counter = cnt + 7;
-      PANN_CUDA(launch_emulate_global(idx, plan, z, c, e2, st));
+      PANN_CUDA(launch_emulate_global(idx, plan, z.e2_slots, c, e2, st));
       return PANN_OK;
     }
     if (phase & TIERS_FIRST)
@@ -641,7 +642,7 @@ int enqueue_tiers(const pann_index* idx, const SearchPlan& plan, const SearchArg
     t.job_list = glist;
     t.njobs_dev = gcount;
     t.job_counter = cnt + 7;
-    PANN_CUDA(launch_emulate_global(idx, plan, z, t, e, st));
+    PANN_CUDA(launch_emulate_global(idx, plan, z.e2_slots, t, e, st));
   }
   return PANN_OK;
 }

@@ -243,11 +243,14 @@ extern "C" int pann_search_device_noalloc(pann_index* idx, const void* d_queries
     e.bits0 = bits0;
     e.vs_slots = vs;
     e.base_bytes = basew;
-    size_t smem_need = emu_smem_bytes(basew, vs, (uint32_t)(4 * S0), (uint32_t)(2 * S0), true);
+    // a block per query where its state and tables fit, else a warp
+    const size_t smem_block =
+        emu_block_layout(idx->stride, plan.L, plan.Ccap, idx->R, vs, (uint32_t)(4 * S0), (uint32_t)(2 * S0)).bytes;
+    const size_t smem_warp = emu_smem_bytes(basew, vs, (uint32_t)(4 * S0), (uint32_t)(2 * S0), true);
     const uint32_t* glist = emu;
     uint32_t* gcount = cnt + 6;
     const uint32_t* grec = emu_rec;
-    if (smem_need <= smem_cap && 4 * S0 < (1ull << 31)) {
+    if (std::min(smem_block, smem_warp) <= smem_cap && 4 * S0 < (1ull << 30)) {
       e.capA = (uint32_t)(4 * S0);
       e.capB = (uint32_t)(2 * S0);
       e.overflow_list = ovf;
@@ -257,7 +260,11 @@ extern "C" int pann_search_device_noalloc(pann_index* idx, const void* d_queries
       t.job_list = emu;
       t.njobs_dev = cnt + 6;
       t.job_counter = cnt + 5;
-      PANN_CUDA(launch_emulate(idx->dtype, idx->metric, true, t, e, 2 * idx->sm_count, smem_need, st));
+      if (smem_block <= smem_cap)
+        PANN_CUDA(launch_emulate_block(idx->dtype, idx->metric, true, t, e, (int)std::min<uint64_t>(idx->sm_count, nq),
+                                       smem_block, st));
+      else
+        PANN_CUDA(launch_emulate(idx->dtype, idx->metric, true, t, e, 2 * idx->sm_count, smem_warp, st));
       glist = ovf;
       grec = ovf_rec;
       gcount = cnt + 8;
@@ -273,7 +280,7 @@ extern "C" int pann_search_device_noalloc(pann_index* idx, const void* d_queries
     t.job_list = glist;
     t.njobs_dev = gcount;
     t.job_counter = cnt + 7;
-    PANN_CUDA(launch_emulate(idx->dtype, idx->metric, false, t, e, e2_slots, emu_smem_bytes(basew, vs, 0, 0, false), st));
+    PANN_CUDA(launch_emulate_global(idx, plan, e2_slots, t, e, st));
   }
   return PANN_OK;
 }

@@ -56,6 +56,9 @@ cudaError_t launch_emulate(int dtype, int metric, bool smem_tables, const Search
 constexpr int EMU_BLOCK_WARPS = 4;
 cudaError_t launch_emulate_block(int dtype, int metric, bool smem_tables, const SearchArgs& a, const EmuArgs& e,
                                  int blocks, size_t smem, cudaStream_t st);
+// The same with the tables in `slots` pairs of global memory (e.gA, e.gB).
+cudaError_t launch_emulate_global(const pann_index* idx, const SearchPlan& plan, int slots, const SearchArgs& a,
+                                  const EmuArgs& e, cudaStream_t st);
 // Tier 0's table, warps and blocks (S_force, wpb_force: 0 = automatic).
 int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
                 int wpb_force, int minb, TierSizes* z);
