@@ -189,7 +189,7 @@ template <int DT, int MT, int SEEN, int PREC = PREC_F32>
 static auto search_kernel_ptr(int minb) {
   if constexpr (SEEN != SEEN_GLOBAL && PREC == PREC_F32)
     if (minb == 4) return search_kernel<DT, MT, SEEN, PREC, 6>;
-  return search_kernel<DT, MT, SEEN, PREC, PREC == PREC_F32 ? 4 : 3>;
+  return search_kernel<DT, MT, SEEN, PREC, 4>;
 }
 
 template <int DT, int MT, int SEEN, int PREC = PREC_F32>
@@ -209,7 +209,8 @@ cudaError_t launch_search(int dtype, int metric, int seen, const SearchArgs& a, 
 #define PANN_LP_CASE(MT, PR)                                                               \
     if (metric == MT && prec == PR)                                                        \
       return seen == SEEN_GLOBAL ? launch_search_t<DT_F32, MT, SEEN_GLOBAL, PR>(a, blocks, threads, smem, st, 3) \
-                                 : launch_search_t<DT_F32, MT, SEEN32, PR>(a, blocks, threads, smem, st, 3);
+             : seen == SEEN16  ? launch_search_t<DT_F32, MT, SEEN16, PR>(a, blocks, threads, smem, st, 3)        \
+                               : launch_search_t<DT_F32, MT, SEEN32, PR>(a, blocks, threads, smem, st, 3);
     PANN_LP_CASE(MT_L2, PREC_BF16)
     PANN_LP_CASE(MT_IP, PREC_BF16)
     PANN_LP_CASE(MT_L2, PREC_FP8)
@@ -316,11 +317,16 @@ static int search_occupancy(int dtype, int metric, int seen, int threads, size_t
   return 0;
 }
 
-static int lp_occupancy(int metric, int prec, int threads, size_t smem) {
-  if (metric == MT_L2 && prec == PREC_BF16) return occupancy_t<DT_F32, MT_L2, SEEN32, PREC_BF16>(threads, smem);
-  if (metric == MT_IP && prec == PREC_BF16) return occupancy_t<DT_F32, MT_IP, SEEN32, PREC_BF16>(threads, smem);
-  if (metric == MT_L2 && prec == PREC_FP8) return occupancy_t<DT_F32, MT_L2, SEEN32, PREC_FP8>(threads, smem);
-  if (metric == MT_IP && prec == PREC_FP8) return occupancy_t<DT_F32, MT_IP, SEEN32, PREC_FP8>(threads, smem);
+static int lp_occupancy(int metric, int prec, int seen, int threads, size_t smem) {
+#define PANN_LPOCC_CASE(MT, PR)                                                                   \
+  if (metric == MT && prec == PR)                                                                 \
+    return seen == SEEN16 ? occupancy_t<DT_F32, MT, SEEN16, PR>(threads, smem)                    \
+                          : occupancy_t<DT_F32, MT, SEEN32, PR>(threads, smem);
+  PANN_LPOCC_CASE(MT_L2, PREC_BF16)
+  PANN_LPOCC_CASE(MT_IP, PREC_BF16)
+  PANN_LPOCC_CASE(MT_L2, PREC_FP8)
+  PANN_LPOCC_CASE(MT_IP, PREC_FP8)
+#undef PANN_LPOCC_CASE
   return 0;
 }
 
@@ -353,7 +359,7 @@ int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int 
   const size_t cap = idx->smem_optin;
   const uint32_t S_min = pow2_at_least(4ull * (idx->R + 1));
   uint32_t S = S_force ? std::max<uint32_t>(pow2_at_least(S_force), S_min) : tier0_slots(plan, idx->R);
-  z->scratch = precision == PREC_F32 ? row_score_scratch_rt(idx->dtype) : 0u;
+  z->scratch = row_score_scratch_rt(idx->dtype);
   uint32_t nbits = 1;
   while (nbits < 31 && (1ull << nbits) < idx->n) nbits++;
   // with at most 12 queries an SM the wider table fits anyway, and probing it takes fewer instructions
@@ -361,7 +367,7 @@ int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int 
   auto shape = [&]() {
     uint32_t sbits = 0;
     while ((1u << sbits) < S) sbits++;
-    z->seen = precision == PREC_F32 && many && nbits <= sbits + SEEN16_REM ? SEEN16 : SEEN32;
+    z->seen = many && nbits <= sbits + SEEN16_REM ? SEEN16 : SEEN32;
     z->id_bits = std::max(nbits, sbits);
     z->wb = search_warp_bytes(idx->stride, plan.L, plan.Ccap, idx->R, S, z->seen, z->scratch);
   };
@@ -383,7 +389,7 @@ int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int 
     if ((size_t)z->wb * w > cap) return 0;
     const int o = precision == PREC_F32
                       ? search_occupancy(idx->dtype, idx->metric, z->seen, 32 * w, (size_t)z->wb * w, minb)
-                      : lp_occupancy(idx->metric, precision, 32 * w, (size_t)z->wb * w);
+                      : lp_occupancy(idx->metric, precision, z->seen, 32 * w, (size_t)z->wb * w);
     return std::max(o, 1);
   };
   int wpb = 0, occ = 0;

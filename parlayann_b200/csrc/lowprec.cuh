@@ -28,65 +28,56 @@ __device__ __forceinline__ float2 e4m3x2_to_f2(uint32_t v) {
   return __half22float2(*reinterpret_cast<__half2*>(&h));
 }
 
-// Approximate distances of up to two low-precision rows to the query staged in
-// shared memory as float32 (negated for L2, as the exact path stores it).
-// FP8 rows are dequantized with the per-dimension scales in shared memory.
+// Adds chunk c (16 bytes) of a low-precision row to the two partial sums of its approximate distance to the query
+// staged in shared memory as float32 (negated for L2, as the exact path stores it). FP8 values are dequantized with
+// the per-dimension scales.
 template <int MT, int PREC>
-__device__ __forceinline__ void lp_dist2(const uint8_t* __restrict__ rowA, const uint8_t* __restrict__ rowB,
-                                         const float* qs, const float* scales, int d, int lp_chunks, float& da,
-                                         float& db) {
-  const bool two = rowB != nullptr;
-  const uint4* ra = reinterpret_cast<const uint4*>(rowA);
-  const uint4* rb = reinterpret_cast<const uint4*>(two ? rowB : rowA);
-  float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-  constexpr int VPC = PREC == PREC_BF16 ? 8 : 16;  // values per 16-byte chunk
-  for (int c0 = 0; c0 < lp_chunks; c0 += 8) {
-    uint4 ba[8], bb[8];
+__device__ __forceinline__ void lp_chunk(const uint4& v, int c, const float* qs, const float* __restrict__ scales, int d,
+                                         float& a0, float& a1) {
+  constexpr int VPC = PREC == PREC_BF16 ? 8 : 16;  // values per chunk
+  const uint32_t wa[4] = {v.x, v.y, v.z, v.w};
+  const int e0 = c * VPC;
 #pragma unroll
-    for (int c = 0; c < 8; c++)
-      if (c0 + c < lp_chunks) {
-        ba[c] = __ldg(ra + c0 + c);
-        bb[c] = two ? __ldg(rb + c0 + c) : make_uint4(0, 0, 0, 0);
+  for (int w = 0; w < 4; w++) {
+#pragma unroll
+    for (int h = 0; h < (PREC == PREC_BF16 ? 1 : 2); h++) {
+      const int e = e0 + w * (VPC / 4) + 2 * h;
+      if (e >= d) break;
+      float2 x;
+      if (PREC == PREC_BF16) {
+        x = bf16x2_to_f2(wa[w]);
+      } else {
+        x = e4m3x2_to_f2(wa[w] >> (16 * h));
+        x.x *= scales[e]; x.y *= scales[e + 1];
       }
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      if (c0 + c >= lp_chunks) break;
-      const uint32_t wa[4] = {ba[c].x, ba[c].y, ba[c].z, ba[c].w};
-      const uint32_t wb[4] = {bb[c].x, bb[c].y, bb[c].z, bb[c].w};
-      const int e0 = (c0 + c) * VPC;
-#pragma unroll
-      for (int w = 0; w < 4; w++) {
-#pragma unroll
-        for (int h = 0; h < (PREC == PREC_BF16 ? 1 : 2); h++) {
-          const int e = e0 + w * (VPC / 4) + 2 * h;
-          if (e >= d) break;
-          float2 xa, xb;
-          if (PREC == PREC_BF16) {
-            xa = bf16x2_to_f2(wa[w]);
-            xb = bf16x2_to_f2(wb[w]);
-          } else {
-            xa = e4m3x2_to_f2(wa[w] >> (16 * h));
-            xb = e4m3x2_to_f2(wb[w] >> (16 * h));
-            xa.x *= scales[e]; xa.y *= scales[e + 1];
-            xb.x *= scales[e]; xb.y *= scales[e + 1];
-          }
-          const float q0 = qs[e], q1 = qs[e + 1];
-          if (MT == MT_L2) {
-            float t;
-            t = xa.x + q0; a0 = fmaf(t, t, a0);
-            t = xa.y + q1; a1 = fmaf(t, t, a1);
-            t = xb.x + q0; b0 = fmaf(t, t, b0);
-            t = xb.y + q1; b1 = fmaf(t, t, b1);
-          } else {
-            a0 = fmaf(q0, xa.x, a0); a1 = fmaf(q1, xa.y, a1);
-            b0 = fmaf(q0, xb.x, b0); b1 = fmaf(q1, xb.y, b1);
-          }
-        }
+      const float q0 = qs[e], q1 = qs[e + 1];
+      if (MT == MT_L2) {
+        float t;
+        t = x.x + q0; a0 = fmaf(t, t, a0);
+        t = x.y + q1; a1 = fmaf(t, t, a1);
+      } else {
+        a0 = fmaf(q0, x.x, a0); a1 = fmaf(q1, x.y, a1);
       }
     }
   }
-  da = MT == MT_L2 ? a0 + a1 : -(a0 + a1);
-  if (two) db = MT == MT_L2 ? b0 + b1 : -(b0 + b1);
+}
+
+// Approximate distance of one low-precision row, eight chunks of it in flight.
+template <int MT, int PREC>
+__device__ __forceinline__ float lp_dist(const uint8_t* __restrict__ row, const float* qs, const float* scales, int d,
+                                         int lp_chunks) {
+  const uint4* ra = reinterpret_cast<const uint4*>(row);
+  float a0 = 0.0f, a1 = 0.0f;
+  for (int c0 = 0; c0 < lp_chunks; c0 += 8) {
+    uint4 b[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (c0 + c < lp_chunks) b[c] = __ldg(ra + c0 + c);
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (c0 + c < lp_chunks) lp_chunk<MT, PREC>(b[c], c0 + c, qs, scales, d, a0, a1);
+  }
+  return MT == MT_L2 ? a0 + a1 : -(a0 + a1);
 }
 
 }  // namespace pann

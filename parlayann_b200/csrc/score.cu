@@ -39,9 +39,8 @@ __global__ void __launch_bounds__(128) score_kernel(const uint8_t* __restrict__ 
     if (PREC == PREC_F32) {
       dv = point_dist<DT, MT>(points + (uint64_t)id * stride, qs, (int)d, (int)nchunks, qq);
     } else {
-      float dummy;
-      lp_dist2<MT, PREC>(lp_rows + (uint64_t)id * lp_stride, nullptr, reinterpret_cast<const float*>(qs), scales,
-                         (int)d, (int)lp_chunks, dv, dummy);
+      dv = lp_dist<MT, PREC>(lp_rows + (uint64_t)id * lp_stride, reinterpret_cast<const float*>(qs), scales, (int)d,
+                             (int)lp_chunks);
     }
     out[(uint64_t)qi * m + j] = dv;
   }

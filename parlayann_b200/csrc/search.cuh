@@ -457,18 +457,19 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
       if (got < 0) got = table_insert(spill, smask, v);
       return got > 0;
     };
+    // the distance of each of the first n lanes' rows
+    auto score = [&](uint32_t id, int n) -> float {
+      if constexpr (PREC == PREC_F32)
+        return warp_score_rows<DT, MT>(a.points, a.stride, (int)a.nchunks, id, n, qs, scr, qq, lane);
+      else
+        return warp_score_lp<MT, PREC>(a.lp_rows, a.lp_stride, (int)a.lp_chunks, id, n,
+                                       reinterpret_cast<const float*>(qs), a.lp_scales, (int)a.d, scr, lane);
+    };
     for (uint32_t b = 0; b < a.n_start; b += 32) {
       const uint32_t s = b + lane;
       const bool ok = s < a.n_start;
       const uint32_t id = ok ? a.starts[s] : PANN_PAD;
-      float dd = 0.0f, dummy;
-      if (PREC == PREC_F32) {
-        dd = warp_score_rows<DT, MT>(a.points, a.stride, (int)a.nchunks, ok ? id : 0u, (int)min(32u, a.n_start - b), qs,
-                                     scr, qq, lane);
-      } else if (ok) {
-        lp_dist2<MT, PREC>(a.lp_rows + (uint64_t)id * a.lp_stride, nullptr, reinterpret_cast<const float*>(qs),
-                           a.lp_scales, (int)a.d, (int)a.lp_chunks, dd, dummy);
-      }
+      const float dd = score(ok ? id : 0u, (int)min(32u, a.n_start - b));
       if (ok) fr[s] = make_key(dd, id);
       seen_insert(id);
       if (handoff && ok) wlog[s] = id;
@@ -599,38 +600,14 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
       // distances; keep those below the cutoff (:176-182)
       cmps += (uint32_t)nnew;
       if ((uint32_t)(cn + nnew) > a.Ccap) { status |= QS_INTERNAL; break; }
-      if (PREC == PREC_F32) {
-        for (int b = 0; b < nnew; b += 32) {
-          const int i0 = b + lane;
-          const uint32_t v0 = i0 < nnew ? nbuf[i0] : 0u;
-          const float d0 = warp_score_rows<DT, MT>(a.points, a.stride, (int)a.nchunks, v0, min(32, nnew - b), qs, scr, qq,
-                                                   lane);
-          const bool keep0 = i0 < nnew && !(d0 >= cutoff);
-          const unsigned m0 = __ballot_sync(FULL, keep0);
-          if (keep0) cand[cn + __popc(m0 & ((1u << lane) - 1))] = make_key(d0, v0);
-          cn += __popc(m0);
-        }
-      } else
-      // two rows per lane per round: rows b+lane and b+32+lane
-      for (int b = 0; b < nnew; b += 64) {
-        const int i0 = b + lane, i1 = b + 32 + lane;
-        float d0 = 0.0f, d1 = 0.0f;
-        uint32_t v0 = 0, v1 = 0;
-        if (i0 < nnew) {
-          v0 = nbuf[i0];
-          v1 = i1 < nnew ? nbuf[i1] : 0u;
-          lp_dist2<MT, PREC>(a.lp_rows + (uint64_t)v0 * a.lp_stride,
-                             i1 < nnew ? a.lp_rows + (uint64_t)v1 * a.lp_stride : nullptr,
-                             reinterpret_cast<const float*>(qs), a.lp_scales, (int)a.d, (int)a.lp_chunks, d0, d1);
-        }
-        bool keep0 = i0 < nnew && !(d0 >= cutoff);
-        unsigned m0 = __ballot_sync(FULL, keep0);
+      for (int b = 0; b < nnew; b += 32) {
+        const int i0 = b + lane;
+        const uint32_t v0 = i0 < nnew ? nbuf[i0] : 0u;
+        const float d0 = score(v0, min(32, nnew - b));
+        const bool keep0 = i0 < nnew && !(d0 >= cutoff);
+        const unsigned m0 = __ballot_sync(FULL, keep0);
         if (keep0) cand[cn + __popc(m0 & ((1u << lane) - 1))] = make_key(d0, v0);
         cn += __popc(m0);
-        bool keep1 = i1 < nnew && !(d1 >= cutoff);
-        unsigned m1 = __ballot_sync(FULL, keep1);
-        if (keep1) cand[cn + __popc(m1 & ((1u << lane) - 1))] = make_key(d1, v1);
-        cn += __popc(m1);
       }
       // deferred batching (:185-192)
       if (cn == 0 || (cn < defer_below && cnt_after >= 1)) continue;
@@ -700,25 +677,17 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
       // (beam_search_rerank's full-precision pass, beamSearch.h:569-587)
       const uint32_t rr = a.rerank ? a.rerank : 4 * kq;  // 0: 4k of this query
       const int nr = (int)min((uint32_t)fn, rr > kq ? rr : kq);
-      for (int b = 0; b < nr; b += 64) {
-        const int i0 = b + lane, i1 = b + 32 + lane;
-        float d0 = 0.f, d1 = 0.f;
-        uint32_t v0 = 0, v1 = 0;
-        if (i0 < nr) {
-          v0 = key_id(fr[i0]);
-          v1 = i1 < nr ? key_id(fr[i1]) : 0u;
-          point_dist2<DT, MT>(a.points + (uint64_t)v0 * a.stride,
-                              i1 < nr ? a.points + (uint64_t)v1 * a.stride : nullptr, qs, a.nchunks, qq, d0, d1,
-                              a.opaque_zero);
-          fr2[i0] = make_key(d0, v0);
-          if (i1 < nr) fr2[i1] = make_key(d1, v1);
-        }
+      for (int b = 0; b < nr; b += 32) {
+        const int i0 = b + lane;
+        const uint32_t v0 = i0 < nr ? key_id(fr[i0]) : 0u;
+        const float d0 = warp_score_rows<DT, MT>(a.points, a.stride, (int)a.nchunks, v0, min(32, nr - b), qs, scr, qq, lane);
+        if (i0 < nr) fr[i0] = make_key(d0, v0);
       }
       __syncwarp();
       for (int i = lane; i < nr; i += 32) {
-        const uint64_t ki = fr2[i];
+        const uint64_t ki = fr[i];
         int r = 0;
-        for (int j = 0; j < nr; j++) r += fr2[j] < ki;
+        for (int j = 0; j < nr; j++) r += fr[j] < ki;
         if ((uint32_t)r < kq) {
           oid[r] = key_id(ki);
           if (odist) odist[r] = key_dist(ki);

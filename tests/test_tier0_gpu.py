@@ -62,3 +62,23 @@ def test_long_frontier(lib_built):
     for L in (1000, 1024, 1100):
         check(idx.search(q, 10, L), O.search("oracle", base, q, g, 10, L))
     idx.close()
+
+
+# low-precision rows of a part of a 16-byte chunk up to several 128-byte column blocks, in 16-bit tables (many queries)
+# and in wider ones (few): the same traversal, and re-ranked distances that are exactly Point::distance
+@pytest.mark.parametrize("d", [1, 7, 16, 17, 33, 129, 300])
+@pytest.mark.parametrize("precision", [P.PREC_BF16, P.PREC_FP8])
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+def test_low_precision_rows(d, precision, metric, lib_built):
+    n, R = 4000, 37
+    base = random_points(np.float32, n, d, d)
+    q = random_points(np.float32, 3000, d, d + 1)
+    idx = P.Index(base, R, metric)
+    idx.set_graph(O.random_graph(n, R, d + 2, min_deg=1))
+    idx.set_precision(precision)
+    many = idx.search(q, 10, 40, precision=precision)
+    few = idx.search(q[:50], 10, 40, precision=precision)
+    for f in ("ids", "dists", "visited", "cmps"):
+        np.testing.assert_array_equal(getattr(many, f)[:50], getattr(few, f))
+    np.testing.assert_array_equal(few.dists, idx.score(q[:50], few.ids))
+    idx.close()
