@@ -15,7 +15,7 @@
 // module's load until the process exits. It holds the per-call counters, the
 // start points, the per-query work lists and status words, a padded copy of
 // the queries when the row size is not a multiple of 16 bytes, the per-warp
-// global seen tables of the large-table tier and the per-warp emulated
+// global seen tables of the large-table tier and the per-block emulated
 // hashsets of the global emulation tier. A call whose layout does not fit is
 // rejected with PANN_EINVAL and a message; nothing is truncated. The tiers run
 // the same kernels as pann_search_device minus two optional buffers (the
