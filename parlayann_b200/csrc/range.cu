@@ -158,7 +158,7 @@ enum : uint32_t {
 // So a round keeps as much in flight as it can: rows, then table slots, eight
 // a thread, without a barrier between them; one pass that places the calls;
 // rows scored 32 a warp (warp_score_rows); a growth on the whole block. 193
-// expansions of ~3,900 answers (200K x 96 float, R 64): 3.4 -> 1.5 ms. A
+// expansions of ~3,900 answers (200K x 96 float, R 64): 3.4 -> 1.4 ms. A
 // round spent 5.6K of its 36K cycles on warp 0 counting the calls, 6K on
 // gathering, 3.4K each on compacting and looking up, 8.5K on the calls and,
 // averaged, 4.5K on growths.

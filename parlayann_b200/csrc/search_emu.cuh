@@ -1142,7 +1142,7 @@ __device__ __forceinline__ int block_merge(const uint64_t* fr, int fn, const uin
 
 // SMEM: both tables in shared memory, else in global memory (slot blockIdx.x
 // of gA and gB), where a visit waits for L2 instead; four warps that score
-// and a block that rebuilds a growing table make up for it (0.46 ms where a
+// and a block that rebuilds a growing table make up for it (0.32 ms where a
 // warp per query took 1.44 ms: batch of 4,000, beams to 400, 200K x 96 float).
 template <int DT, int MT, int NW, int CH, bool SMEM>
 __global__ void __launch_bounds__(NW * 32, 1) search_emulate_block_kernel(SearchArgs a, EmuArgs e) {
