@@ -24,58 +24,13 @@
 #include "index.cuh"
 #include "lowprec.cuh"
 #include "rowscore.cuh"
+#include "tile_layout.cuh"
 #include "tiers.cuh"
 #include "umma.cuh"
 
 namespace pann {
 
 enum : uint32_t { QS_TRUNCATED = 32u };  // the seen table filled: the search stopped early
-
-struct TileLayout {
-  size_t q, sc, fr, fr2, cand, cid, table, stage, misc, qb, nrm, tcw, total;
-  uint32_t sstride;  // staged row stride (bytes; CUDA-core scoring)
-};
-
-// Rows a tensor-core scoring round takes: the MMA's M.
-constexpr uint32_t TC_ROWS = 128;
-
-// CW: candidates a step can produce (parents x degree); CWs: rows staged at
-// once (a step with more candidates stages and scores them in rounds). With
-// tensor-core scoring (tc) the rows are staged TC_ROWS at a time in the
-// core-matrix layout (umma.cuh), beside the query operand (16 rows: the
-// query's split terms, the rest zero), the staged rows' squared norms and the
-// MMA barrier and tensor-memory address.
-__host__ __device__ inline TileLayout tile_layout(uint32_t d, uint32_t L, uint32_t CW, uint32_t S,
-                                                  uint64_t lp_stride, uint32_t CWs, bool tc = false) {
-  TileLayout t{};
-  size_t o = 0;
-  const size_t dpad = (d + 15) & ~15u;  // whole 16-byte chunks of the low-precision row, of either type
-  // rows at an odd multiple of 16 bytes apart: conflict-free 16-byte reads
-  t.sstride = (uint32_t)(((lp_stride / 16) % 2 == 0) ? lp_stride + 16 : lp_stride);
-  // every region starts on a 16-byte boundary (cp.async destinations and MMA operands need it)
-#define PANN_TILE_TAKE(field, bytes) \
-  t.field = o;                        \
-  o += ((size_t)(bytes) + 15) & ~(size_t)15;
-  PANN_TILE_TAKE(q, 4 * dpad)
-  PANN_TILE_TAKE(sc, 4 * dpad)
-  PANN_TILE_TAKE(fr, 8ull * L)
-  PANN_TILE_TAKE(fr2, 8ull * L)
-  PANN_TILE_TAKE(cand, 8ull * (CW > L ? CW : L))
-  PANN_TILE_TAKE(cid, 4ull * CW)
-  PANN_TILE_TAKE(table, 4ull * S)
-  if (tc) {
-    PANN_TILE_TAKE(stage, (size_t)TC_ROWS * lp_stride)
-    PANN_TILE_TAKE(qb, 16 * lp_stride)
-    PANN_TILE_TAKE(nrm, 4ull * TC_ROWS)
-    PANN_TILE_TAKE(tcw, 16)
-  } else {
-    PANN_TILE_TAKE(stage, (size_t)CWs * t.sstride)
-  }
-  PANN_TILE_TAKE(misc, 64)
-#undef PANN_TILE_TAKE
-  t.total = o;
-  return t;
-}
 
 __device__ __forceinline__ uint64_t fma2_rn(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
@@ -136,19 +91,6 @@ __device__ __forceinline__ float tile_row_dist(const uint8_t* row, const float* 
   }
   const float r = __uint_as_float((uint32_t)acc) + __uint_as_float((uint32_t)(acc >> 32));
   return MT == MT_L2 ? r : -r;
-}
-
-// Seen-set slots of a query with beam L: (L + 16) * nel * 1.35 rounded up to
-// a multiple of 32, within [4 (R + 1), 16384] (not a power of two: slots are
-// chosen by multiplicative range reduction); a query stops early (flagged) when
-// its set reaches 15/16 of that. Per query, so a batch answers each query as a
-// search with that query's beam alone would.
-__host__ __device__ inline uint32_t tile_seen_slots(uint32_t L, uint32_t nel, uint32_t R) {
-  uint64_t s = ((uint64_t)(L + 16) * nel * 135 / 100 + 31) & ~31ull;
-  const uint64_t lo = 4ull * (R + 1);
-  if (s < lo) s = (lo + 31) & ~31ull;
-  if (s > 16384) s = 16384;
-  return (uint32_t)s;
 }
 
 // Home slot in [0, S) of an id (Fibonacci hashing, then range reduction).
@@ -483,22 +425,20 @@ __global__ void __launch_bounds__(128, 6) search_tile_kernel(SearchArgs a, uint3
     const uint32_t rr = a.rerank ? a.rerank : 4 * kq;
     const uint32_t nr = fn < (rr > kq ? rr : kq) ? fn : (rr > kq ? rr : kq);
     {
-      // the seen table and the stage are free now: the query as the exact kernels stage it, then row buffers for as
-      // many warps as fit (rowscore.cuh); without one, a row per thread
-      uint8_t* const qs = smem + ly.table;
-      const uint32_t qb = (uint32_t)((a.stride + 15) & ~15ull);
-      const uint32_t room = (uint32_t)((TC ? ly.qb : ly.misc) - ly.table);
-      const uint32_t nwarp = room > qb ? min(4u, (room - qb) / row_score_scratch<DT_F32>()) : 0u;
-      for (uint32_t i = tid; i < (uint32_t)a.stride / 4; i += blockDim.x) {
-        const float x = i < a.d ? qf[i] : 0.0f;
-        reinterpret_cast<float*>(qs)[i] = MT == MT_L2 ? -x : x;
-      }
+      // the query in place as the exact kernels stage it (its padding is zero); row buffers over the seen table and the
+      // stage, which are free now, for as many warps as fit (rowscore.cuh); without one, a row per thread
+      const TileRerank rr_ly = tile_rerank(ly, TC, row_score_scratch<DT_F32>());
+      const uint8_t* const qs = smem + rr_ly.q;
+      const uint32_t nwarp = rr_ly.warps;
+      if (MT == MT_L2)
+        for (uint32_t i = tid; i < ((a.d + 15) & ~15u); i += blockDim.x) qf[i] = -qf[i];
       __syncthreads();
       if (nwarp > 0) {
         for (uint32_t b = 32 * warp; (uint32_t)warp < nwarp && b < nr; b += 32 * nwarp) {
           const uint32_t id = b + lane < nr ? key_id(fr[b + lane]) : 0u;
+          uint8_t* const stg = smem + rr_ly.scratch + warp * row_score_scratch<DT_F32>();
           const float dd = warp_score_rows<DT_F32, MT>(a.points, a.stride, (int)a.nchunks, id, (int)min(32u, nr - b),
-                                                       qs, qs + qb + warp * row_score_scratch<DT_F32>(), 0, lane);
+                                                       qs, stg, 0, lane);
           if (b + lane < nr) cand[b + lane] = make_key(dd, id);
         }
       } else {
