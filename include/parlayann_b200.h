@@ -467,7 +467,10 @@ int pann_build(pann_index* idx, const pann_build_params* bp, const uint32_t* per
 
 /* Exact top-k by full scan (data_tools/compute_groundtruth.cpp:22-60):
  * integer types in exact integer arithmetic, float in FP64. Ties ordered by id.
- * Host buffers; out_dists may be NULL. */
+ * Host buffers; out_dists may be NULL. Works in buffers of its own (up to
+ * 768 MB stay with the index between calls, larger ones go back), so it may
+ * run beside searches and a server on the same index; calls of this function
+ * on one index, from several threads, take turns. */
 int pann_groundtruth(pann_index* idx, const void* queries, uint32_t nq, uint32_t k, uint32_t* out_ids,
                      double* out_dists);
 

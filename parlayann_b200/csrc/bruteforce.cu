@@ -263,13 +263,20 @@ extern "C" int pann_groundtruth(pann_index* idx, const void* queries, uint32_t n
   size_t rb = (size_t)idx->d * idx->esize;
   size_t smem = 8 * idx->stride + 8 * (size_t)k * (sizeof(double) + sizeof(uint32_t));
   if (smem > idx->smem_optin) return fail(PANN_EINVAL, "k too large for the brute-force kernel");
-  // the index's resident buffers
-  PANN_CUDA(idx->q.ensure(idx->stride * (size_t)nq));
-  PANN_CUDA(idx->ids.ensure(4ull * k * nq));
-  PANN_CUDA(idx->dists.ensure(8ull * k * nq));
-  uint8_t* dq = idx->q.as<uint8_t>();
-  uint32_t* dids = idx->ids.as<uint32_t>();
-  double* dd = idx->dists.as<double>();
+  std::lock_guard<std::mutex> lock(idx->gt_mu);
+  struct Bounded {  // buffers past GT_KEEP go back when the call ends
+    pann_index* idx;
+    ~Bounded() {
+      for (DevBuf* b : {&idx->gt_io, &idx->gt})
+        if (b->bytes > GT_KEEP) b->release();
+    }
+  } bounded{idx};
+  // distances, queries, ids
+  const size_t o_q = (8ull * k * nq + 255) & ~size_t(255), o_ids = o_q + ((idx->stride * (size_t)nq + 255) & ~size_t(255));
+  PANN_CUDA(idx->gt_io.ensure(o_ids + 4ull * k * nq));
+  double* dd = idx->gt_io.as<double>();
+  uint8_t* dq = idx->gt_io.as<uint8_t>() + o_q;
+  uint32_t* dids = reinterpret_cast<uint32_t*>(idx->gt_io.as<uint8_t>() + o_ids);
   if (rb != idx->stride) PANN_CUDA(cudaMemsetAsync(dq, 0, idx->stride * (size_t)nq, st));
   PANN_CUDA(cudaMemcpy2DAsync(dq, idx->stride, queries, rb, rb, nq, cudaMemcpyHostToDevice, st));
   // the tensor-core path; the plain kernel takes what it does not: k above 256, rows too long for its shared

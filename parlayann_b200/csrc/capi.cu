@@ -927,6 +927,7 @@ int pann_index_destroy(pann_index* idx) {
     b->release();
   idx->lp_norms.release();
   idx->order.release();
+  idx->gt_io.release();
   idx->gt.release();
   if (idx->ev_fork) cudaEventDestroy(idx->ev_fork);
   if (idx->ev_join) cudaEventDestroy(idx->ev_join);

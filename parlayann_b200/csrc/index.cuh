@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include "../../include/parlayann_b200.h"
 
@@ -93,7 +94,10 @@ struct pann_index {
   int32_t q_offset = 0;
   float q_bound = 1.0f;  // mips: the trimmed bound
   bool graph_borrowed = false;  // d_graph belongs to another index
-  pann::DevBuf gt;  // brute-force groundtruth workspace: operand images and candidate buffers (gt_tensor.cu), bounded
+  // brute-force groundtruth: queries and results; operand images and candidate buffers (gt_tensor.cu). Its own, so that
+  // it runs beside searches; one call at a time, GT_KEEP bytes of each kept between calls
+  std::mutex gt_mu;
+  pann::DevBuf gt_io, gt;
   uint32_t starts_cached_n = 0;
   uint32_t starts_cached[64] = {};
 };

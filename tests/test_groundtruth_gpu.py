@@ -1,5 +1,8 @@
 """Exact top-k on the tensor cores (csrc/gt_tensor.cu) against the plain FP64 / integer kernel, which answers the
 same call with PANN_GT_PLAIN set: ids and distances equal bit for bit (both are exact, ties by id)."""
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 
@@ -59,3 +62,48 @@ def test_float_scales(lib_built, monkeypatch):
     want = both(base, q, 10, P.L2, monkeypatch)
     np.testing.assert_array_equal(ids, want[0])
     np.testing.assert_array_equal(dd, want[1])
+
+
+def test_beside_searches_and_other_threads(lib_built):
+    """Groundtruth calls of two threads beside device searches of padded rows on a third stream, all on one index."""
+    import torch
+
+    from oracle import oracle as O
+
+    n, d, R, nq, k, L = 20000, 7, 24, 3000, 10, 60
+    base, q = random_points(np.float32, n, d, 1), random_points(np.float32, nq, d, 2)
+    idx = P.Index(base, R)
+    idx.set_graph(O.random_graph(n, R, 3, min_deg=16))
+    dq = torch.from_numpy(q).cuda()
+    want = idx.search(q, k, L)
+    parts = [(q[:700], 20), (q[700:1900], 5)]
+    alone = [idx.groundtruth(*p) for p in parts]
+    got = [[], []]
+
+    def gt(i):
+        for _ in range(12):
+            got[i].append(idx.groundtruth(*parts[i]))
+
+    ids = [torch.zeros((nq, k), dtype=torch.int32, device="cuda") for _ in range(12)]
+    dists = [torch.zeros((nq, k), dtype=torch.float32, device="cuda") for _ in range(12)]
+    flags = torch.zeros(nq, dtype=torch.int32, device="cuda")
+    stream, qp, start = torch.cuda.Stream(), P.QueryParams(k, L, n, R, 0.125), np.zeros(1, np.uint32)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=gt, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for i in range(12):
+        rc = P.lib().pann_search_device(idx.handle, dq.data_ptr(), nq, ctypes.byref(qp), start.ctypes.data, 1,
+                                        ids[i].data_ptr(), dists[i].data_ptr(), None, None, flags.data_ptr(),
+                                        stream.cuda_stream)
+        assert rc == 0
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(12):
+        np.testing.assert_array_equal(ids[i].cpu().numpy().view(np.uint32), want.ids)
+        np.testing.assert_array_equal(dists[i].cpu().numpy(), want.dists)
+        for part in range(2):
+            np.testing.assert_array_equal(got[part][i][0], alone[part][0])
+            np.testing.assert_array_equal(got[part][i][1], alone[part][1])
+    idx.close()
