@@ -24,15 +24,17 @@ namespace pann {
 
 template <int DT, int MT>
 __global__ void __launch_bounds__(256) bruteforce_kernel(const uint8_t* __restrict__ points, uint64_t n, uint64_t stride,
-                                                         int d, const uint8_t* __restrict__ queries, uint32_t nq,
-                                                         uint32_t k, uint32_t* out_ids, double* out_d) {
+                                                         int d, const uint8_t* __restrict__ queries,
+                                                         const uint32_t* __restrict__ list, uint32_t nq, uint32_t k,
+                                                         uint32_t* out_ids, double* out_d) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t qi = blockIdx.x * 8 + warp;
+  const uint32_t at = blockIdx.x * 8 + warp;
+  const bool active = at < nq;
+  const uint32_t qi = list && active ? list[at] : at;
   uint8_t* qs = smem + (size_t)warp * stride;
   double* bd = reinterpret_cast<double*>(smem + 8 * stride) + (size_t)warp * k;
   uint32_t* bi = reinterpret_cast<uint32_t*>(reinterpret_cast<double*>(smem + 8 * stride) + 8 * (size_t)k) + (size_t)warp * k;
-  const bool active = qi < nq;
   if (active)
     for (uint64_t c = lane; c < stride / 16; c += 32)
       reinterpret_cast<uint4*>(qs)[c] = reinterpret_cast<const uint4*>(queries + (uint64_t)qi * stride)[c];
@@ -213,28 +215,17 @@ extern "C" int pann_range_groundtruth(pann_index* idx, const void* queries, uint
   return PANN_OK;
 }
 
-// The queries of `list` by the plain kernel, scattered into dids / dd.
-static int groundtruth_plain(pann_index* idx, const uint8_t* dq, const std::vector<uint32_t>& list, uint32_t k,
+// The nf queries of the device array `list` (NULL: the first nf) by the plain kernel, in place: rows read from dq,
+// answers written to dids / dd at the query's own rows.
+static int groundtruth_plain(pann_index* idx, const uint8_t* dq, const uint32_t* list, uint32_t nf, uint32_t k,
                              uint32_t* dids, double* dd, cudaStream_t st) {
-  const uint32_t nf = (uint32_t)list.size();
-  struct Owned : DevBuf {
-    ~Owned() { release(); }
-  };
-  Owned fq, fids, fd;
-  PANN_CUDA(fq.ensure(idx->stride * (size_t)nf));
-  PANN_CUDA(fids.ensure(4ull * k * nf));
-  PANN_CUDA(fd.ensure(8ull * k * nf));
-  for (uint32_t i = 0; i < nf; i++)
-    PANN_CUDA(cudaMemcpyAsync(fq.as<uint8_t>() + (size_t)i * idx->stride, dq + (size_t)list[i] * idx->stride,
-                              idx->stride, cudaMemcpyDeviceToDevice, st));
   const size_t smem = 8 * idx->stride + 8 * (size_t)k * (sizeof(double) + sizeof(uint32_t));
-#define PANN_BF_CASE(DT, MT)                                                                                     \
-  if (idx->dtype == DT && idx->metric == MT) {                                                                   \
-    auto kern = bruteforce_kernel<DT, MT>;                                                                       \
-    PANN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max()));         \
-    kern<<<(nf + 7) / 8, 256, smem, st>>>(idx->d_points, idx->n, idx->stride, (int)idx->d, fq.as<uint8_t>(), nf, \
-                                          k, fids.as<uint32_t>(), fd.as<double>());                              \
-    PANN_CUDA(cudaGetLastError());                                                                               \
+#define PANN_BF_CASE(DT, MT)                                                                                           \
+  if (idx->dtype == DT && idx->metric == MT) {                                                                         \
+    auto kern = bruteforce_kernel<DT, MT>;                                                                             \
+    PANN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max()));               \
+    kern<<<(nf + 7) / 8, 256, smem, st>>>(idx->d_points, idx->n, idx->stride, (int)idx->d, dq, list, nf, k, dids, dd); \
+    PANN_CUDA(cudaGetLastError());                                                                                     \
   }
   PANN_BF_CASE(DT_U8, MT_L2)
   PANN_BF_CASE(DT_U8, MT_IP)
@@ -243,13 +234,6 @@ static int groundtruth_plain(pann_index* idx, const uint8_t* dq, const std::vect
   PANN_BF_CASE(DT_F32, MT_L2)
   PANN_BF_CASE(DT_F32, MT_IP)
 #undef PANN_BF_CASE
-  for (uint32_t i = 0; i < nf; i++) {
-    PANN_CUDA(cudaMemcpyAsync(dids + (size_t)list[i] * k, fids.as<uint32_t>() + (size_t)i * k, 4ull * k,
-                              cudaMemcpyDeviceToDevice, st));
-    PANN_CUDA(cudaMemcpyAsync(dd + (size_t)list[i] * k, fd.as<double>() + (size_t)i * k, 8ull * k,
-                              cudaMemcpyDeviceToDevice, st));
-  }
-  PANN_CUDA(cudaStreamSynchronize(st));
   return PANN_OK;
 }
 
@@ -271,9 +255,9 @@ extern "C" int pann_groundtruth(pann_index* idx, const void* queries, uint32_t n
         if (b->bytes > GT_KEEP) b->release();
     }
   } bounded{idx};
-  // distances, queries, ids
+  // distances, queries, ids, the queries left to the plain kernel
   const size_t o_q = (8ull * k * nq + 255) & ~size_t(255), o_ids = o_q + ((idx->stride * (size_t)nq + 255) & ~size_t(255));
-  PANN_CUDA(idx->gt_io.ensure(o_ids + 4ull * k * nq));
+  PANN_CUDA(idx->gt_io.ensure(o_ids + 4ull * k * nq + 4ull * nq));
   double* dd = idx->gt_io.as<double>();
   uint8_t* dq = idx->gt_io.as<uint8_t>() + o_q;
   uint32_t* dids = reinterpret_cast<uint32_t*>(idx->gt_io.as<uint8_t>() + o_ids);
@@ -287,11 +271,13 @@ extern "C" int pann_groundtruth(pann_index* idx, const void* queries, uint32_t n
     rc = groundtruth_tensor(idx, dq, nq, k, dids, dd, &rest, st);
     if (rc != PANN_OK && rc != PANN_EINVAL) return rc;
   }
-  if (rc == PANN_EINVAL) {
-    rest.resize(nq);
-    for (uint32_t i = 0; i < nq; i++) rest[i] = i;
+  const bool all = rc == PANN_EINVAL || rest.size() == nq;
+  if (all || !rest.empty()) {
+    uint32_t* list = all ? nullptr : dids + (size_t)k * nq;
+    if (list) PANN_CUDA(cudaMemcpyAsync(list, rest.data(), 4 * rest.size(), cudaMemcpyHostToDevice, st));
+    rc = groundtruth_plain(idx, dq, list, all ? nq : (uint32_t)rest.size(), k, dids, dd, st);
+    if (rc != PANN_OK) return rc;
   }
-  if (!rest.empty() && (rc = groundtruth_plain(idx, dq, rest, k, dids, dd, st)) != PANN_OK) return rc;
   PANN_CUDA(cudaMemcpyAsync(out_ids, dids, 4ull * k * nq, cudaMemcpyDeviceToHost, st));
   if (out_dists) PANN_CUDA(cudaMemcpyAsync(out_dists, dd, 8ull * k * nq, cudaMemcpyDeviceToHost, st));
   PANN_CUDA(cudaStreamSynchronize(st));

@@ -34,7 +34,7 @@ __device__ __forceinline__ bool dless(double a, uint32_t ia, double b, uint32_t 
   return a < b || (a == b && ia < ib);
 }
 
-// Bytes of each groundtruth buffer that an index keeps between calls. 10K queries on 1M x 96 floats use 265 MB of images
+// Bytes of each groundtruth buffer that an index keeps between calls. 10K queries on 1M x 96 floats use 201 MB of images
 // and candidate buffers; freeing and allocating them would add to every call.
 constexpr size_t GT_KEEP = 384ull << 20;
 

@@ -107,3 +107,30 @@ def test_beside_searches_and_other_threads(lib_built):
             np.testing.assert_array_equal(got[part][i][0], alone[part][0])
             np.testing.assert_array_equal(got[part][i][1], alone[part][1])
     idx.close()
+
+
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+def test_half_of_the_queries_left_to_the_plain_kernel(metric, lib_built, monkeypatch):
+    """Every second query lies near 3,000 copies of one point, whose equal scores its margin test cannot tell apart."""
+    rng = np.random.default_rng(11)
+    base = rng.standard_normal((20000, 24)).astype(np.float32)
+    base[9000:12000] = 3 * base[5]
+    q = rng.standard_normal((201, 24)).astype(np.float32)
+    q[::2] = 3 * base[5] + np.float32(1e-3) * q[::2]
+    both(base, q, 15, metric, monkeypatch)
+
+
+def test_plain_kernel_works_in_place(lib_built):
+    """k above 256 goes to the plain kernel whole. 4,000 queries on 300 points take it about 3 ms; a copy of each
+    query's row, ids and distances (12,000 copies) would take at least 12 ms at 1 us a copy."""
+    import time
+
+    idx = P.Index(random_points(np.float32, 300, 16, 1), 4)
+    q = random_points(np.float32, 4000, 16, 2)
+    times = []
+    for _ in range(6):
+        t = time.perf_counter()
+        idx.groundtruth(q, 257)
+        times.append(time.perf_counter() - t)
+    idx.close()
+    assert min(times) < 12e-3, times
