@@ -3,15 +3,21 @@
 // point) pair are one matrix product, computed by tcgen05.mma, and only the
 // pairs below a per-query threshold leave the tensor memory.
 //
-//   gt_absmax_kernel  (float) the largest |value|, which fixes a power-of-two
-//                     scale into half precision's range
+//   gt_centre_kernel  (float) a centre c for data far from the origin, else
+//                     zero: distances and the order of dot products with one
+//                     query do not change when c is taken off every point
+//                     (and, Euclidean, off the queries), the norms that the
+//                     error margin grows with do
+//   gt_absmax_kernel  (float) the largest |value - c|, which fixes a
+//                     power-of-two scale into half precision's range
 //   gt_image_kernel   operand images: tiles of rows laid out in global memory
 //                     exactly as the MMA reads them from shared memory (8-row
 //                     x 16-byte core matrices, 64 bytes of K at a time), so a
 //                     tile is fetched with plain bulk copies. 8-bit rows are
-//                     copied; a float row x is split into two half-precision
-//                     planes, hi = fp16(x s) and lo = fp16(x s - hi), which
-//                     hold x s to 2^-24 relative (half a float32 ulp).
+//                     copied; a float row x (less c) is split into two
+//                     half-precision planes, hi = fp16(x s) and lo =
+//                     fp16(x s - hi), which hold x s to 2^-23 relative (one
+//                     float32 ulp: the rest after hi has up to 13 bits, lo 11).
 //   gt_mma_kernel     one block per (N queries, slice of the points): the
 //                     queries' image stays in shared memory, point tiles of
 //                     128 rows stream through a ring of bulk copies, one
@@ -28,21 +34,25 @@
 //                     float: FP64 distances of the candidates within the
 //                     scores' error margin decide, ties by id.
 //
-// Float margin: |score - exact| <= bound with u = 2^-24, B = max |b| and
-//   split        hi + lo misses x s by at most u |x s|, or 2^-25 (half of the
-//                smallest step) where the value is 2^-14 or less of the
-//                largest, which adds 2^-37 sqrt(d) B (|q| + the batch's largest
-//                value); lo.lo <= u |q||b| is left out: 4 u |q||b|
+// Float margin: |score - exact| <= bound with u = 2^-24, b and q the rows less
+// c, B = max |b|; first-order sums:
+//   centre       b and q are rounded differences, u |b| and u |q| off: moves
+//                |b|^2 - 2 q.b by 2 u B^2 + 4 u |q| B (q.b by u |q| B)
+//   split        hi + lo misses x s by at most 2 u |x s|, or 2^-25 (half of the
+//                smallest step) where lo is below half precision's normal range,
+//                which moves a dot product by at most 2^-38 sqrt(d) B (|q| + the
+//                batch's largest value); lo.lo <= 4 u |q||b| is left out: 8 u |q||b|
 //   accumulation 3 d products, each addition off by at most 2 u |q||b| (the
 //                tensor core may truncate): 6 d u |q||b|
-//   |b|^2 and the final FMA: u B^2 each and u of the result
-// so bound = 2 (2 u B^2 + 2 (6 d + 8) u |q| B) for Euclidean distance and
-// 2 (6 d + 8) u |q| B for mips (plus the step term), twice the first-order
-// sums. A true top-k
-// point has score <= s_k + 2 bound (s_k: the k-th smallest score); if the
+//   |b|^2 and the final FMA: u B^2 and u of the result, u (B^2 + 2 |q| B) or u |q| B
+// The sums are 4 u B^2 + 2 (6 d + 11) u |q| B for Euclidean distance and
+// (6 d + 10) u |q| B for mips (plus the step term); bound is twice that. A true
+// top-k point has score <= s_k + 2 bound (s_k: the k-th smallest score); if the
 // query's threshold is above that, no slice dropped such a point. A query
 // that fails the test (or whose survivors do not fit) is left to the plain
-// kernel.
+// kernel, which is about 80 times slower: without a centre that were all
+// queries of unit-variance data 32 from the origin in each of 96 dimensions
+// (100K points, 1,000 queries: 51 ms; 0.62 ms with it, as at the origin).
 //
 // What bounds it (10K queries x 1M x 96 floats, k 20; 120 ms with float32
 // FMAs on the CUDA cores, 8.4 ms here): the three products are 5.8 TFLOP of
@@ -75,8 +85,9 @@ constexpr uint32_t GT_FCAP = 1024;     // float candidates scored in FP64
 constexpr double GT_HUGE = 1e15;
 
 struct GtScale {
-  uint32_t pt_max, q_max;            // bits of the largest |value| (float)
+  uint32_t pt_max, q_max;            // bits of the largest |value - c| (float)
   unsigned long long bmax;           // bits of the largest |b| (double)
+  uint32_t centre_done;              // blocks of gt_centre_kernel that have finished
 };
 
 __device__ __forceinline__ int gt_exp(uint32_t max_bits) {
@@ -88,13 +99,118 @@ __device__ __forceinline__ int gt_exp(uint32_t max_bits) {
   return min(14 - e, 120);
 }
 
-__global__ void gt_absmax_kernel(const uint4* __restrict__ rows, uint64_t nchunks, uint32_t* out) {
-  uint32_t m = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nchunks; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint4 v = __ldg(rows + i);
-    const uint32_t w[4] = {v.x & 0x7FFFFFFFu, v.y & 0x7FFFFFFFu, v.z & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu};
+// The centre: the mean of a sample of the points (any centre is valid; 512
+// rows bring it within a 22nd of the spread), taken where it holds at least
+// three quarters of the sample's mean square, so that B falls to about half or
+// less; nearer the origin the points' spread sets B and zero costs no rounding.
+// A block per 32 columns and 32 rows, four loads a thread in flight; the last
+// one to finish adds the partial sums (always in the same order) and decides.
+constexpr uint32_t GT_CEN_ROWS = 512, GT_CEN_PARTS = 16;
+struct GtCentre {
+  double *sum, *sq;  // GT_CEN_PARTS rows of cols
+  uint32_t* cnt;
+  float* centre;     // cols
+  uint32_t cols;
+};
+__global__ void __launch_bounds__(256) gt_centre_kernel(const uint8_t* __restrict__ points, uint64_t stride, uint64_t n,
+                                                        GtCentre g, GtScale* sc) {
+  __shared__ double s_a[8][32], s_b[8][32];
+  __shared__ uint32_t s_c[8][32];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t col = blockIdx.x * 32 + lane;
+  const uint32_t m = (uint32_t)min(n, (uint64_t)GT_CEN_ROWS);
+  const uint64_t step = n / m * stride;
+  constexpr int PER = GT_CEN_ROWS / GT_CEN_PARTS / 8;
+  float x[PER];
 #pragma unroll
-    for (int j = 0; j < 4; j++) m = w[j] < 0x7F800000u && w[j] > m ? w[j] : m;  // finite values only
+  for (int t = 0; t < PER; t++) {
+    const uint32_t r = (blockIdx.y * PER + t) * 8 + warp;
+    x[t] = r < m && col < g.cols ? __ldg(reinterpret_cast<const float*>(points + r * step) + col) : __int_as_float(0x7fffffff);
+  }
+  double sum = 0.0, sq = 0.0;
+  uint32_t cnt = 0;
+#pragma unroll
+  for (int t = 0; t < PER; t++)
+    if (fabsf(x[t]) < __int_as_float(0x7f800000)) {  // finite values only
+      sum += (double)x[t];
+      sq += (double)x[t] * (double)x[t];
+      cnt++;
+    }
+  s_a[warp][lane] = sum;
+  s_b[warp][lane] = sq;
+  s_c[warp][lane] = cnt;
+  __syncthreads();
+  if (warp == 0) {
+    for (int w = 1; w < 8; w++) {
+      sum += s_a[w][lane];
+      sq += s_b[w][lane];
+      cnt += s_c[w][lane];
+    }
+    if (col < g.cols) {
+      const uint32_t at = blockIdx.y * g.cols + col;
+      g.sum[at] = sum;
+      g.sq[at] = sq;
+      g.cnt[at] = cnt;
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) s_last = atomicAdd(&sc->centre_done, 1u) == gridDim.x * gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double c2 = 0.0, m2 = 0.0;  // squared norm of the mean, mean squared norm
+  for (uint32_t j = threadIdx.x; j < g.cols; j += blockDim.x) {
+    double a = 0.0, b = 0.0;
+    uint32_t c = 0;
+#pragma unroll
+    for (uint32_t p = 0; p < GT_CEN_PARTS; p++) {
+      a += __ldcg(g.sum + p * g.cols + j);
+      b += __ldcg(g.sq + p * g.cols + j);
+      c += __ldcg(g.cnt + p * g.cols + j);
+    }
+    const float mean = c ? (float)(a / c) : 0.0f;
+    g.centre[j] = mean;
+    c2 += (double)mean * (double)mean;
+    m2 += c ? b / c : 0.0;
+  }
+  for (int o = 16; o; o >>= 1) {
+    c2 += __shfl_xor_sync(0xFFFFFFFFu, c2, o);
+    m2 += __shfl_xor_sync(0xFFFFFFFFu, m2, o);
+  }
+  if (lane == 0) {
+    s_a[0][warp] = c2;
+    s_b[0][warp] = m2;
+  }
+  __syncthreads();
+  c2 = m2 = 0.0;
+  for (int w = 0; w < 8; w++) {
+    c2 += s_a[0][w];
+    m2 += s_b[0][w];
+  }
+  if (c2 >= 0.75 * m2) return;
+  for (uint32_t j = threadIdx.x; j < g.cols; j += blockDim.x) g.centre[j] = 0.0f;
+}
+
+// Rows of rowchunks 16-byte chunks each; centre: a row of the same length, or NULL.
+__global__ void gt_absmax_kernel(const float4* __restrict__ rows, uint64_t nchunks, uint32_t rowchunks,
+                                 const float4* __restrict__ centre, uint32_t* out) {
+  uint32_t m = 0;
+  const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+  uint32_t j = (uint32_t)(first % rowchunks);
+  const uint32_t jstep = (uint32_t)(step % rowchunks);
+  for (uint64_t i = first; i < nchunks; i += step) {
+    const float4 v = __ldg(rows + i);
+    const float4 c = centre ? __ldg(centre + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float x[4] = {__fsub_rn(v.x, c.x), __fsub_rn(v.y, c.y), __fsub_rn(v.z, c.z), __fsub_rn(v.w, c.w)};
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const uint32_t w = __float_as_uint(x[t]) & 0x7FFFFFFFu;
+      m = w < 0x7F800000u && w > m ? w : m;  // finite values only
+    }
+    j += jstep;
+    if (j >= rowchunks) j -= rowchunks;
   }
   m = __reduce_max_sync(0xFFFFFFFFu, m);
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
@@ -107,8 +223,9 @@ __global__ void gt_absmax_kernel(const uint4* __restrict__ rows, uint64_t nchunk
 template <int DT>
 __global__ void __launch_bounds__(256) gt_image_kernel(const uint8_t* __restrict__ rows, uint64_t stride, uint32_t d,
                                                        uint64_t nrows, uint64_t rows_total, uint32_t tile_rows,
-                                                       uint32_t kch, const GtScale* sc, int is_query, uint8_t* img,
-                                                       void* norms, unsigned long long* bmax) {
+                                                       uint32_t kch, const GtScale* sc, const float4* __restrict__ centre,
+                                                       int is_query, uint8_t* img, void* norms,
+                                                       unsigned long long* bmax) {
   const int lane = threadIdx.x & 31;
   const int r8 = lane >> 2, c = lane & 3;
   const uint32_t planes = DT == DT_F32 ? 2 : 1;
@@ -132,7 +249,8 @@ __global__ void __launch_bounds__(256) gt_image_kernel(const uint8_t* __restrict
           const uint32_t b = kc * 128 + c * 32 + q * 16;  // byte of the row
           if (row < nrows && b < stride) {
             const float4 v = __ldg(reinterpret_cast<const float4*>(src + b));
-            const float x[4] = {v.x, v.y, v.z, v.w};
+            const float4 c4 = centre ? __ldg(centre + b / 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float x[4] = {__fsub_rn(v.x, c4.x), __fsub_rn(v.y, c4.y), __fsub_rn(v.z, c4.z), __fsub_rn(v.w, c4.w)};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
               n2 += (double)x[j] * (double)x[j];
@@ -664,10 +782,11 @@ __global__ void __launch_bounds__(GT_FT) gt_final_kernel(GtFinal g) {
       const double u = 5.9604644775390625e-08;  // 2^-24
       const double qn = sqrt((double)reinterpret_cast<const float*>(g.qnorm)[qi]) * (1.0 + 1e-6);
       const double B = __longlong_as_double((long long)g.scale->bmax) * (1.0 + 1e-6);
-      // 2^-37 sqrt(d): half precision's smallest step below the batch's (the points') largest value
+      // 2^-37 sqrt(d): half precision's smallest step below the batch's (the points') largest value, twice
       const double step = 7.275957614183426e-12 * sqrt((double)g.d);
-      const double acc = ((6.0 * g.d + 8.0) * u * qn + step * ((double)__uint_as_float(g.scale->q_max) + qn)) * B;
-      const double bound = MT == MT_L2 ? 2.0 * (2.0 * u * B * B + 2.0 * acc) + 1e-12 : 2.0 * acc + 1e-12;
+      const double acc = ((6.0 * g.d + (MT == MT_L2 ? 11.0 : 10.0)) * u * qn +
+                          step * ((double)__uint_as_float(g.scale->q_max) + qn)) * B;
+      const double bound = MT == MT_L2 ? 2.0 * (4.0 * u * B * B + 2.0 * acc) + 1e-12 : 2.0 * acc + 1e-12;
       lim = (double)float_of(v) + 2.0 * bound;
       const bool cut = thr != 0xFFFFFFFFu;  // no slice dropped anything otherwise
       bad = !(qn < GT_HUGE && B < GT_HUGE) || (cut && !((double)float_of(thr) > lim)) || !(lim == lim);
@@ -750,16 +869,14 @@ static cudaError_t gt_launch_mma(const GtMma& g, uint32_t qtiles, size_t smem, c
 
 template <int DT, int MT>
 static cudaError_t gt_run_dm(const pann_index* idx, GtMma m, GtFinal f, uint32_t qtiles, uint64_t seg_rows,
-                             uint8_t* a_img, void* pnorm, GtScale* sc, size_t smem_mma, size_t smem_fin,
-                             cudaStream_t st) {
-  const uint32_t PL = DT == DT_F32 ? 2 : 1;
-  (void)PL;
+                             uint8_t* a_img, void* pnorm, GtScale* sc, const float4* centre, size_t smem_mma,
+                             size_t smem_fin, cudaStream_t st) {
   for (uint64_t r0 = 0; r0 < idx->n; r0 += seg_rows) {
     const uint64_t rows = std::min<uint64_t>(seg_rows, idx->n - r0);
     const uint64_t total = (rows + GT_ROWS - 1) / GT_ROWS * GT_ROWS;
     gt_image_kernel<DT><<<(int)std::min<uint64_t>((total / 8 + 7) / 8, 16ull * idx->sm_count), 256, 0, st>>>(
-        idx->d_points + r0 * idx->stride, idx->stride, idx->d, rows, total, GT_ROWS, m.kch, sc, 0, a_img, pnorm,
-        &sc->bmax);
+        idx->d_points + r0 * idx->stride, idx->stride, idx->d, rows, total, GT_ROWS, m.kch, sc, centre, 0, a_img,
+        pnorm, &sc->bmax);
     m.n_seg = (uint32_t)rows;
     m.ntiles = (uint32_t)(total / GT_ROWS);
     m.id0 = (uint32_t)r0;
@@ -814,7 +931,8 @@ int groundtruth_tensor(pann_index* idx, const uint8_t* dq, uint32_t nq, uint32_t
   const size_t o_sc = take(sizeof(GtScale) + 64), o_a = take(seg * row_img), o_pn = take(4 * seg),
                o_b = take((size_t)qtiles * N * row_img), o_qn = take(4ull * qtiles * N),
                o_cand = take(8ull * qc * slices * CB), o_cnt = take(4ull * qc * slices), o_thr = take(4ull * qc),
-               o_fb = take(4ull * qc);
+               o_fb = take(4ull * qc), o_cen = take(F ? idx->stride : 0),
+               o_part = take(F ? 5ull * GT_CEN_PARTS * idx->stride : 0);
   PANN_CUDA(idx->gt.ensure(o));
   uint8_t* w = idx->gt.as<uint8_t>();
   GtScale* sc = reinterpret_cast<GtScale*>(w + o_sc);
@@ -825,23 +943,32 @@ int groundtruth_tensor(pann_index* idx, const uint8_t* dq, uint32_t nq, uint32_t
     PANN_CUDA(cudaMemsetAsync(w + o_sc, 0, sizeof(GtScale) + 64, st));
     PANN_CUDA(cudaMemsetAsync(w + o_cnt, 0, 4ull * qc * slices, st));
     PANN_CUDA(cudaMemsetAsync(w + o_thr, 0xFF, 4ull * qc, st));
+    const float4* centre = F ? reinterpret_cast<const float4*>(w + o_cen) : nullptr;
+    const float4* qcentre = idx->metric == MT_L2 ? centre : nullptr;
     if (F) {
-      gt_absmax_kernel<<<4 * idx->sm_count, 256, 0, st>>>(reinterpret_cast<const uint4*>(idx->d_points),
-                                                          idx->n * idx->nchunks, &sc->pt_max);
-      gt_absmax_kernel<<<idx->sm_count, 256, 0, st>>>(reinterpret_cast<const uint4*>(q), (uint64_t)nc * idx->nchunks,
-                                                      &sc->q_max);
+      GtCentre gc;
+      gc.cols = (uint32_t)(idx->stride / 4);
+      gc.sum = reinterpret_cast<double*>(w + o_part);
+      gc.sq = gc.sum + (size_t)GT_CEN_PARTS * gc.cols;
+      gc.cnt = reinterpret_cast<uint32_t*>(gc.sq + (size_t)GT_CEN_PARTS * gc.cols);
+      gc.centre = reinterpret_cast<float*>(w + o_cen);
+      gt_centre_kernel<<<dim3((gc.cols + 31) / 32, GT_CEN_PARTS), 256, 0, st>>>(idx->d_points, idx->stride, idx->n, gc, sc);
+      gt_absmax_kernel<<<4 * idx->sm_count, 256, 0, st>>>(reinterpret_cast<const float4*>(idx->d_points),
+                                                          idx->n * idx->nchunks, idx->nchunks, centre, &sc->pt_max);
+      gt_absmax_kernel<<<idx->sm_count, 256, 0, st>>>(reinterpret_cast<const float4*>(q), (uint64_t)nc * idx->nchunks,
+                                                      idx->nchunks, qcentre, &sc->q_max);
     }
     const uint64_t qtotal = (uint64_t)qtiles * N;
     const int qb = (int)std::min<uint64_t>((qtotal / 8 + 7) / 8, 16ull * idx->sm_count);
     if (F)
-      gt_image_kernel<DT_F32><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, 1, w + o_b, w + o_qn,
-                                                  nullptr);
+      gt_image_kernel<DT_F32><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, qcentre, 1, w + o_b,
+                                                  w + o_qn, nullptr);
     else if (idx->dtype == DT_U8)
-      gt_image_kernel<DT_U8><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, 1, w + o_b, w + o_qn,
-                                                 nullptr);
+      gt_image_kernel<DT_U8><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, nullptr, 1, w + o_b,
+                                                 w + o_qn, nullptr);
     else
-      gt_image_kernel<DT_I8><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, 1, w + o_b, w + o_qn,
-                                                 nullptr);
+      gt_image_kernel<DT_I8><<<qb, 256, 0, st>>>(q, idx->stride, idx->d, nc, qtotal, N, kch, sc, nullptr, 1, w + o_b,
+                                                 w + o_qn, nullptr);
     PANN_CUDA(cudaGetLastError());
     GtMma m{};
     m.a_img = w + o_a;
@@ -882,7 +1009,7 @@ int groundtruth_tensor(pann_index* idx, const uint8_t* dq, uint32_t nq, uint32_t
     const uint32_t qt = (nc + N - 1) / N;
 #define PANN_GT_CASE(DT, MT)                                                                                       \
     if (idx->dtype == DT && idx->metric == MT)                                                                     \
-      e = gt_run_dm<DT, MT>(idx, m, f, qt, seg, w + o_a, w + o_pn, sc, smem_mma, smem_fin, st);
+      e = gt_run_dm<DT, MT>(idx, m, f, qt, seg, w + o_a, w + o_pn, sc, centre, smem_mma, smem_fin, st);
     PANN_GT_CASE(DT_U8, MT_L2)
     PANN_GT_CASE(DT_U8, MT_IP)
     PANN_GT_CASE(DT_I8, MT_L2)

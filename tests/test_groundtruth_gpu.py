@@ -134,3 +134,48 @@ def test_plain_kernel_works_in_place(lib_built):
         times.append(time.perf_counter() - t)
     idx.close()
     assert min(times) < 12e-3, times
+
+
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+@pytest.mark.parametrize("d,offset", [(1, 1000), (33, 40), (96, 3000)])
+def test_far_from_the_origin(d, offset, metric, lib_built, monkeypatch):
+    """Points around a centre many spreads from the origin, some values not finite."""
+    base = random_points(np.float32, 5000, d, d) + np.float32(offset)
+    q = random_points(np.float32, 130, d, d + 1) + np.float32(offset)
+    both(base, q, 10, metric, monkeypatch)
+    base[::500, d // 2] = np.nan
+    both(base[1:], q, 10, metric, monkeypatch)
+
+
+def test_far_from_the_origin_takes_the_same_path(lib_built):
+    """A common offset does not send queries to the plain kernel, which takes some 45 times as long for these sizes."""
+    import time
+
+    base, q = random_points(np.float32, 100_000, 32, 1), random_points(np.float32, 1000, 32, 2)
+    best = []
+    for offset in (0, 64):
+        idx = P.Index(base + np.float32(offset), 4)
+        times = []
+        for _ in range(6):
+            t = time.perf_counter()
+            idx.groundtruth(q + np.float32(offset), 20)
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+        idx.close()
+    assert best[1] < 5 * best[0], best
+
+
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+def test_values_that_half_precision_splits_worst(metric, lib_built, monkeypatch):
+    """Values 1 + j 2^-23 with odd j in (2048, 4096): the rest after the upper half has 13 bits, the lower half holds 11,
+    so both halves miss the value by a whole float32 ulp. Random signs keep the mean at the origin; the distances of the
+    points that share a query's signs differ in their last bits."""
+    rng = np.random.default_rng(12)
+    d = 40
+
+    def rows(sign):
+        j = 2 * rng.integers(1024, 2048, sign.shape) + 1
+        return (sign * (1 + j * 2.0 ** -23)).astype(np.float32)
+
+    sign = rng.choice([-1.0, 1.0], (100, d))
+    both(rows(np.repeat(sign, 30, 0)), rows(sign), 20, metric, monkeypatch)
