@@ -26,7 +26,7 @@
 //                     two alternating accumulators, and sixteen warps read
 //                     the finished one: score = |b|^2 - 2 q.b (or -q.b), kept if
 //                     below the query's threshold. A kept pair goes to the
-//                     (query, slice) buffer; a buffer of more than C + 64 keys
+//                     (query, slice) buffer; a buffer of more than C + GT_CUT keys
 //                     is cut to about C, the last of whose scores is a
 //                     threshold for every slice of that query.
 //   gt_final_kernel   a block per query: the surviving keys of all slices;
@@ -79,7 +79,8 @@ constexpr int GT_EPI_WARPS = 16;         // four a scheduler: with two the epilo
 constexpr int GT_THREADS = 32 * (GT_EPI_WARPS + 2);
 constexpr int GT_COLS = 256 / GT_EPI_WARPS;    // thresholds a warp keeps
 constexpr uint64_t GT_WAIT_NS = 4000000000ull;  // a wait this long means a lost arrival
-constexpr uint32_t GT_CAP = 12288;     // surviving keys a query's final block takes
+constexpr uint32_t GT_CUT = 64;        // a buffer of more than C + GT_CUT keys is cut
+constexpr uint32_t GT_CAP = 12288;     // slices x C, at most: the final kernel's scores take up to twice as many words
 constexpr uint32_t GT_FCAP = 1024;     // float candidates scored in FP64
 // scores above this could overflow float32 on the way: the plain kernel takes over
 constexpr double GT_HUGE = 1e15;
@@ -635,9 +636,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gt_mma_kernel(GtMma g) {
       if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
       __syncwarp();
       epi_barrier();  // every append of this tile is in its buffer
-      // a buffer is cut at C + 64 keys (so it can take a whole tile: CB is at least C + 64 + GT_ROWS): a cut
+      // a buffer is cut at C + GT_CUT keys (so it can take a whole tile: CB is at least C + GT_CUT + GT_ROWS): a cut
       // costs about as much as eight appends, and the sooner the threshold falls the fewer there are
-      unsigned cut = __ballot_sync(FULL, col_live && cnt_s[mycol] > g.C + 64);
+      unsigned cut = __ballot_sync(FULL, col_live && cnt_s[mycol] > g.C + GT_CUT);
       while (cut) {
         const int j = __ffs(cut) - 1;
         cut &= cut - 1;
@@ -703,28 +704,52 @@ __device__ __forceinline__ uint32_t gt_block_sum(uint32_t n, uint32_t* red) {
   return s;
 }
 
+// Survivors are the keys at or below the query's threshold, the smallest of
+// the slices' own; a slice holds at most C + GT_CUT keys when its last tile is
+// done, so their scores (a word each) fit in `cap` = slices x (C + GT_CUT)
+// words whatever the data. The k-th smallest score is found on those words and
+// the keys it selects are read again from the buffers (in L2). Whole keys in a
+// block of GT_CAP overflowed with many slices, by the order of the appends: 100
+// queries on 300K x 96 floats, k 100, 0.9 or 68 ms; 0.84 ms always now.
 template <int DT, int MT>
 __global__ void __launch_bounds__(GT_FT) gt_final_kernel(GtFinal g) {
   extern __shared__ __align__(16) uint8_t fsm[];
   __shared__ uint32_t s_n, s_red[GT_FT / 32], s_m;
   constexpr bool F = DT == DT_F32;
-  uint64_t* keys = reinterpret_cast<uint64_t*>(fsm);
+  uint32_t* words = reinterpret_cast<uint32_t*>(fsm + (F ? 12u * GT_FCAP : 8u * g.k));
   const uint32_t qi = blockIdx.x, tid = threadIdx.x;
   const uint32_t thr = g.thr[qi];
   if (tid == 0) { s_n = 0; s_m = 0; }
   __syncthreads();
-  // survivors: at or below the query's threshold
-  for (uint32_t s = 0; s < g.slices; s++) {
-    const uint64_t slot = (uint64_t)qi * g.slices + s;
-    const uint32_t c = g.count[slot];
-    for (uint32_t i = tid; i < c; i += GT_FT) {
-      const uint64_t key = g.cand[slot * g.CB + i];
-      if ((uint32_t)(key >> 32) <= thr) {
-        const uint32_t p = atomicAdd(&s_n, 1u);
-        if (p < g.cap) keys[p] = key;
+  // every key of the query's buffers: a warp takes every fourth slice, four keys a lane in flight (the passes wait for
+  // L2; slice after slice on the whole block they took 43 us at 148 slices)
+  auto each_key = [&](auto&& use) {
+    constexpr uint32_t NW = GT_FT / 32;
+    const uint32_t lane = tid & 31, warp = tid >> 5;
+    const uint32_t* cq = g.count + (uint64_t)qi * g.slices;
+    for (uint32_t s0 = 0; s0 < g.slices; s0 += GT_FT) {
+      const uint32_t mine = s0 + NW * lane + warp;
+      const uint32_t cnt = mine < g.slices ? cq[mine] : 0u;
+      for (uint32_t l = 0; l < 32 && s0 + NW * l + warp < g.slices; l++) {
+        const uint32_t c = __shfl_sync(0xFFFFFFFFu, cnt, l);
+        const uint64_t* keys = g.cand + ((uint64_t)qi * g.slices + s0 + NW * l + warp) * g.CB;
+        for (uint32_t i = lane; i < c; i += 128) {
+          uint64_t k[4];
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) k[j] = i + 32 * j < c ? keys[i + 32 * j] : ~0ull;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++)
+            if (i + 32 * j < c) use(k[j]);
+        }
       }
     }
-  }
+  };
+  each_key([&](uint64_t key) {
+    if ((uint32_t)(key >> 32) <= thr) {
+      const uint32_t p = atomicAdd(&s_n, 1u);
+      if (p < g.cap) words[p] = (uint32_t)(key >> 32);
+    }
+  });
   __syncthreads();
   const uint32_t m = s_n;
   bool bad = m > g.cap || m < g.k;
@@ -733,7 +758,7 @@ __global__ void __launch_bounds__(GT_FT) gt_final_kernel(GtFinal g) {
     for (int b = 31; b >= 0; b--) {
       const uint32_t t = v | ((1u << b) - 1u);
       uint32_t n = 0;
-      for (uint32_t i = tid; i < m; i += GT_FT) n += (uint32_t)(keys[i] >> 32) <= t;
+      for (uint32_t i = tid; i < m; i += GT_FT) n += words[i] <= t;
       if (gt_block_sum(n, s_red) < g.k) v |= 1u << b;
     }
   }
@@ -742,29 +767,35 @@ __global__ void __launch_bounds__(GT_FT) gt_final_kernel(GtFinal g) {
     if (!bad) {
       uint32_t less = 0, eq = 0;
       for (uint32_t i = tid; i < m; i += GT_FT) {
-        less += (uint32_t)(keys[i] >> 32) < v;
-        eq += (uint32_t)(keys[i] >> 32) == v;
+        less += words[i] < v;
+        eq += words[i] == v;
       }
       less = gt_block_sum(less, s_red);
       eq = gt_block_sum(eq, s_red);
       uint32_t idmax = 0x7FFFFFFFu;
-      if (less + eq > g.k) {
+      if (less + eq > g.k) {  // the ids at that score, in place of the scores
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        each_key([&](uint64_t key) {
+          if ((uint32_t)(key >> 32) == v) words[atomicAdd(&s_n, 1u)] = (uint32_t)key;
+        });
+        __syncthreads();
         idmax = 0;
         for (int b = 30; b >= 0; b--) {
           const uint32_t t = idmax | ((1u << b) - 1u);
           uint32_t n = 0;
-          for (uint32_t i = tid; i < m; i += GT_FT) n += (uint32_t)(keys[i] >> 32) == v && (uint32_t)keys[i] <= t;
+          for (uint32_t i = tid; i < eq; i += GT_FT) n += words[i] <= t;
           if (gt_block_sum(n, s_red) < g.k - less) idmax |= 1u << b;
         }
       }
-      uint64_t* best = keys + g.cap;
-      for (uint32_t i = tid; i < m; i += GT_FT) {
-        const uint32_t h = (uint32_t)(keys[i] >> 32);
-        if (h < v || (h == v && (uint32_t)keys[i] <= idmax)) {
+      uint64_t* best = reinterpret_cast<uint64_t*>(fsm);
+      each_key([&](uint64_t key) {
+        const uint32_t h = (uint32_t)(key >> 32);
+        if (h < v || (h == v && (uint32_t)key <= idmax)) {
           const uint32_t p = atomicAdd(&s_m, 1u);
-          if (p < g.k) best[p] = keys[i];
+          if (p < g.k) best[p] = key;
         }
-      }
+      });
       __syncthreads();
       const long long qn = MT == MT_L2 ? (long long)reinterpret_cast<const int32_t*>(g.qnorm)[qi] : 0ll;
       for (uint32_t i = tid; i < g.k; i += GT_FT) {
@@ -791,14 +822,16 @@ __global__ void __launch_bounds__(GT_FT) gt_final_kernel(GtFinal g) {
       const bool cut = thr != 0xFFFFFFFFu;  // no slice dropped anything otherwise
       bad = !(qn < GT_HUGE && B < GT_HUGE) || (cut && !((double)float_of(thr) > lim)) || !(lim == lim);
     }
-    uint32_t* idv = reinterpret_cast<uint32_t*>(keys + g.cap);
-    double* d64 = reinterpret_cast<double*>(idv + GT_FCAP);
+    double* d64 = reinterpret_cast<double*>(fsm);
+    uint32_t* idv = reinterpret_cast<uint32_t*>(d64 + GT_FCAP);
     if (!bad)
-      for (uint32_t i = tid; i < m; i += GT_FT)
-        if ((double)float_of((uint32_t)(keys[i] >> 32)) <= lim) {
+      each_key([&](uint64_t key) {
+        const uint32_t h = (uint32_t)(key >> 32);
+        if (h <= thr && (double)float_of(h) <= lim) {
           const uint32_t p = atomicAdd(&s_m, 1u);
-          if (p < GT_FCAP) idv[p] = (uint32_t)keys[i];
+          if (p < GT_FCAP) idv[p] = (uint32_t)key;
         }
+      });
     __syncthreads();
     const uint32_t nc = s_m;
     bad = bad || nc > GT_FCAP;
@@ -903,7 +936,7 @@ int groundtruth_tensor(pann_index* idx, const uint8_t* dq, uint32_t nq, uint32_t
   // float: the margin test needs room above the k-th score; 8-bit scores are exact
   const uint32_t need = F ? std::max<uint32_t>(64, 2 * k) : std::max<uint32_t>(64, k);
   if (need > 512 || idx->n > 0x7FFFFFFFull - GT_ROWS) return PANN_EINVAL;
-  const uint32_t CB = need <= 64 ? 256 : need <= 256 ? 448 : 704;  // C + 64 + a tile
+  const uint32_t CB = need <= 64 ? 256 : need <= 256 ? 448 : 704;  // C + GT_CUT + a tile
   const uint32_t C = need;
   // point images in segments of at most 128 MB, queries in chunks whose buffers stay within 128 MB
   const uint64_t row_img = (uint64_t)kch * PL * GT_KB;
@@ -919,8 +952,8 @@ int groundtruth_tensor(pann_index* idx, const uint8_t* dq, uint32_t nq, uint32_t
   }
   const uint32_t qtiles = (qc + N - 1) / N;
   const size_t smem_mma = gt_layout(N, kch, PL, stages).total;
-  const uint32_t cap = std::min<uint32_t>(GT_CAP, slices * CB);
-  const size_t smem_fin = 8ull * cap + (F ? 12ull * GT_FCAP : 8ull * k);
+  const uint32_t cap = slices * (C + GT_CUT);
+  const size_t smem_fin = 4ull * cap + (F ? 12ull * GT_FCAP : 8ull * k);
   // workspace
   size_t o = 0;
   auto take = [&](size_t b) {

@@ -179,3 +179,26 @@ def test_values_that_half_precision_splits_worst(metric, lib_built, monkeypatch)
 
     sign = rng.choice([-1.0, 1.0], (100, d))
     both(rows(np.repeat(sign, 30, 0)), rows(sign), 20, metric, monkeypatch)
+
+
+@pytest.mark.parametrize("dtype,d,k", [(np.float32, 256, 100), (np.uint8, 96, 200)])
+def test_survivors_of_many_slices(dtype, d, k, lib_built, monkeypatch):
+    """Few queries on many points are split into slices whose survivors number more than slices x C; they all fit, so
+    the call does not fall back to the plain kernel (measured 25 to 300 times as long for these sizes)."""
+    import time
+
+    base, q = random_points(dtype, 300_000, d, 1), random_points(dtype, 100, d, 2)
+    idx = P.Index(base, 4)
+    took, answers = [], []
+    for plain in ("", "", "", "1"):
+        if plain:
+            monkeypatch.setenv("PANN_GT_PLAIN", plain)
+        t = time.perf_counter()
+        answers.append(idx.groundtruth(q, k))
+        took.append(time.perf_counter() - t)
+    monkeypatch.delenv("PANN_GT_PLAIN")
+    idx.close()
+    for ids, dd in answers[:3]:
+        np.testing.assert_array_equal(ids, answers[3][0])
+        np.testing.assert_array_equal(dd, answers[3][1])
+    assert max(took[1:3]) < took[3] / 5, took
