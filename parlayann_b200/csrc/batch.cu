@@ -104,9 +104,13 @@ static int enqueue(pann_batch* b, const TierSizes& z, cudaStream_t st) {
 // Picks how the batch maps onto the GPU by timing each candidate on the
 // staged batch (three runs each, the first warming the caches, the faster of
 // the other two counts). Every candidate gives the same answers:
+//  * the automatic mapping, which another has to beat by more than 1 % (runs
+//    of one mapping differ by that much);
 //  * exact search, warp per query: the first tier's seen-table slots
-//    ({1/2, 1, 2} x the estimate), warps per block ({2, 4}) and register
-//    budget (fitted to 3 or 4 resident blocks);
+//    ({1/2, 1, 2} x the automatic ones), warps per block ({2, 4} and the
+//    automatic count: 1 to 3 where few queries are spread over the SMs),
+//    entry width (16 bits, and 32 where few queries take them) and register
+//    budget (fitted to four or six resident blocks);
 //  * exact search, CTA per query: every query on one block of the
 //    exact-emulation kernel (when its tables fit in shared memory);
 //  * tile search (precision form, parents > 0): the rows staged and scored per
@@ -122,18 +126,23 @@ static int autotune(pann_batch* b, cudaStream_t st) {
     const uint32_t cw = std::max<uint32_t>(1, std::min<uint32_t>(b->parents, 4)) * std::min(b->plan.dl, b->idx->R);
     for (uint32_t f : {4u, 3u, 2u, 1u}) cands.push_back({b->z, std::max<uint32_t>(16, cw * f / 4)});
   } else {
+    cands.push_back({b->z, 0});
     const uint32_t base_S = b->z.S;
     const uint32_t floor_S = 4 * (b->idx->R + 1);
     for (uint32_t S : {base_S / 2, base_S, base_S * 2})
-      for (int w : {2, 4})
-        for (int minb : {3, 4}) {
-          if (S < floor_S || S > 16384) continue;
-          if (minb == 4 && b->prec != PREC_F32) continue;
-          TierSizes z;
-          if (size_tiers(b->idx, b->plan, b->max_q, b->prec, S, w, &z, minb) != PANN_OK) continue;
-          if (z.S != S || z.wpb != w) continue;  // did not fit as asked
-          cands.push_back({z, 0});
-        }
+      for (int w : {2, 4, b->z.wpb})
+        for (int minb : {3, 4})
+          for (bool width_by_nq : {false, true}) {
+            if (S < floor_S || S > 16384) continue;
+            if (minb == 4 && b->prec != PREC_F32) continue;
+            TierSizes z;
+            if (size_tiers(b->idx, b->plan, b->max_q, b->prec, S, w, &z, minb, width_by_nq) != PANN_OK) continue;
+            if (z.S != S || z.wpb != w) continue;  // did not fit as asked
+            bool known = false;
+            for (const Cand& c : cands)
+              known |= c.z.S == z.S && c.z.wpb == z.wpb && c.z.minb == z.minb && c.z.seen == z.seen && c.z.blocks == z.blocks;
+            if (!known) cands.push_back({z, 0});
+          }
     if (b->prec == PREC_F32 && b->z.emu_smem) {
       TierSizes z = b->z;
       z.cta = true;
@@ -143,7 +152,7 @@ static int autotune(pann_batch* b, cudaStream_t st) {
   cudaEvent_t e0, e1;
   PANN_CUDA(cudaEventCreate(&e0));
   PANN_CUDA(cudaEventCreate(&e1));
-  float best = 1e30f;
+  float best = 1e30f, first = 0.0f;
   Cand best_c{b->z, b->tile_rows};
   int rc = PANN_OK;
   for (auto& c : cands) {
@@ -160,11 +169,13 @@ static int autotune(pann_batch* b, cudaStream_t st) {
       if (rep > 0) t_min = std::min(t_min, ms);  // the first run warms the caches
     }
     if (rc) break;
+    if (&c == &cands[0]) first = t_min;
     if (t_min < best) {
       best = t_min;
       best_c = c;
     }
   }
+  if (!tile && best > 0.99f * first) best_c = cands[0];
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;

@@ -355,7 +355,7 @@ uint32_t tier0_slots(const SearchPlan& p, uint32_t R) {
 // alone on an SM has its L1 and issue slots to itself); many take the count
 // that leaves the most warps resident.
 int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
-                int wpb_force, int minb, TierSizes* z) {
+                int wpb_force, int minb, TierSizes* z, bool width_by_nq) {
   const size_t cap = idx->smem_optin;
   const uint32_t S_min = pow2_at_least(4ull * (idx->R + 1));
   uint32_t S = S_force ? std::max<uint32_t>(pow2_at_least(S_force), S_min) : tier0_slots(plan, idx->R);
@@ -363,7 +363,7 @@ int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int 
   uint32_t nbits = 1;
   while (nbits < 31 && (1ull << nbits) < idx->n) nbits++;
   // with at most 12 queries an SM the wider table fits anyway, and probing it takes fewer instructions
-  const bool many = S_force != 0 || wpb_force != 0 || nq > 12ull * idx->sm_count;
+  const bool many = (!width_by_nq && (S_force != 0 || wpb_force != 0)) || nq > 12ull * idx->sm_count;
   auto shape = [&]() {
     uint32_t sbits = 0;
     while ((1u << sbits) < S) sbits++;
@@ -419,13 +419,13 @@ int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int 
 // global table per warp; (E) queries on which the reference's hashset grows,
 // re-run with that hashset emulated exactly.
 int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
-               int wpb_force, TierSizes* z, int minb_force) {
+               int wpb_force, TierSizes* z, int minb_force, bool width_by_nq) {
   const size_t smem_cap = idx->smem_optin;
   TierSizes& t = *z;
   t = TierSizes{};
   // ---- tier 0
   t.minb = precision == PREC_F32 ? (minb_force == 4 || (minb_force == 0 && t0_minb() == 4) ? 4 : 3) : 3;
-  int rc0 = tier0_shape(idx, plan, nq, precision, S_force, wpb_force, t.minb, &t);
+  int rc0 = tier0_shape(idx, plan, nq, precision, S_force, wpb_force, t.minb, &t, width_by_nq);
   if (rc0) return rc0;
   const uint32_t S = t.S;
   uint32_t Sg = std::max<uint32_t>(4 * S, pow2_at_least(2ull * plan.ref_half));

@@ -59,15 +59,16 @@ cudaError_t launch_emulate_block(int dtype, int metric, bool smem_tables, const 
 // The same with the tables in `slots` pairs of global memory (e.gA, e.gB).
 cudaError_t launch_emulate_global(const pann_index* idx, const SearchPlan& plan, int slots, const SearchArgs& a,
                                   const EmuArgs& e, cudaStream_t st);
-// Tier 0's table, warps and blocks (S_force, wpb_force: 0 = automatic).
+// Tier 0's table, warps and blocks (S_force, wpb_force: 0 = automatic). A forced shape takes 16-bit entries where the
+// ids fit, unless width_by_nq: then the number of queries decides, as in an automatic one.
 int tier0_shape(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
-                int wpb_force, int minb, TierSizes* z);
+                int wpb_force, int minb, TierSizes* z, bool width_by_nq = false);
 uint32_t tier0_slots(const SearchPlan& p, uint32_t R);
 
 // S_force / wpb_force (0 = automatic) override the tier-0 seen-table slots and
 // warps per block.
 int size_tiers(const pann_index* idx, const SearchPlan& plan, uint64_t nq, int precision, uint32_t S_force,
-               int wpb_force, TierSizes* z, int minb_force = 0);
+               int wpb_force, TierSizes* z, int minb_force = 0, bool width_by_nq = false);
 // phase: the first tier, the tiers after it (on the first one's counters and
 // lists, untouched since), or both.
 // side (optional): the index's side stream; the exact-emulation tier then

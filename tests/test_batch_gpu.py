@@ -230,3 +230,25 @@ def test_growth_with_tables_in_global_memory(dtype, d, beam, lib_built):
     check(b.run(q, 10, beam), o, "batch")
     b.close()
     idx.close()
+
+
+def test_autotune_of_small_batches_can_keep_the_automatic_mapping(lib_built):
+    """Batches of few queries are spread over the SMs, one warp a block. That mapping is among the candidates, so some
+    of these sizes keep it (a candidate of two or four warps has to be more than 1 % faster); the answers are the plain
+    search's. The beam is too long for a CTA per query."""
+    base = P.synth_mixture(P.F32, 50_000, 96, 16, 5, 0, sigma=0.3, normalize=True)
+    q = P.synth_mixture(P.F32, 32, 96, 16, 5, 1, sigma=0.3, normalize=True)
+    idx = P.Index(base, 32)
+    idx.build(64, 1.2)
+    warps = []
+    for nq in (1, 2, 3, 5, 8, 16, 32):
+        want = idx.search(q[:nq], 10, 200)
+        b = idx.batch(nq, 10, 200, autotune=True)
+        check(b.run(q[:nq], 10, 200), dict(ids=want.ids, dists=want.dists, visited=want.visited, cmps=want.cmps,
+                                           hash_grew=want.flags), nq)
+        cfg = b.config()
+        assert not cfg["cta_per_query"]
+        warps.append(cfg["warps_per_block"])
+        b.close()
+    idx.close()
+    assert 1 in warps, warps
