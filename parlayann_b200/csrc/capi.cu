@@ -1099,9 +1099,11 @@ int pann_search(pann_index* idx, const void* queries, uint32_t nq, const pann_qu
                       d_cmps, d_status, nullptr, 0, st, 0, 0, 0, 0, phase);
   };
   if (words <= 65536) {
-    // few queries seldom need the later tiers: they are launched only if the first one's counters ask for them
-    // (four launches of about 4 us each behind a single query's search)
-    const bool first_only = nq <= 64;
+    // few queries seldom need the later tiers: they are launched only if the first one's counters ask for them. Saves
+    // 10 to 14 us where no hashset grows (100K x 128 uint8, beam 20: one query 128 -> 117 us, 32 queries 150 -> 139),
+    // costs 17 us where one does (a second wait, no emulation beside the first tier; beam 50: 508 -> 525). Of four sets
+    // none grew up to 8 queries, one at 16, two at 32, three at 64, where it no longer pays
+    const bool first_only = nq <= 32;
     std::vector<uint32_t> h(words + 16);
     rc = run(first_only ? TIERS_FIRST : TIERS_ALL);
     if (rc) return rc;

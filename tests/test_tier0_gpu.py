@@ -82,3 +82,24 @@ def test_low_precision_rows(d, precision, metric, lib_built):
         np.testing.assert_array_equal(getattr(many, f)[:50], getattr(few, f))
     np.testing.assert_array_equal(few.dists, idx.score(q[:50], few.ids))
     idx.close()
+
+
+@pytest.mark.parametrize("nq", [1, 2, 31, 32, 33, 64, 65])
+def test_few_queries_with_growth(nq, lib_built):
+    """Host calls on either side of the size up to which the later tiers are launched only when asked for, on queries
+    of which some make the reference's hashset grow."""
+    base = random_points(np.uint8, 20000, 8, 1)
+    g = O.random_graph(20000, 64, 3, min_deg=60)
+    q = random_points(np.uint8, 300, 8, 2)
+    grew = O.search("oracle", base, q, g, 10, 40)["hash_grew"] > 0
+    assert grew.any() and not grew.all()
+    q = np.concatenate([q[grew], q[~grew]])[:nq]  # the first ones grow
+    idx = P.Index(base, 64)
+    idx.set_graph(g)
+    o = O.search("oracle", base, q, g, 10, 40)
+    r = idx.search(q, 10, 40)
+    check(r, o)
+    np.testing.assert_array_equal(r.flags == 1, o["hash_grew"] > 0)
+    r = idx.search(q[-1:], 10, 40)  # a call after one that grew
+    check(r, O.search("oracle", base, q[-1:], g, 10, 40))
+    idx.close()
