@@ -202,3 +202,11 @@ def test_survivors_of_many_slices(dtype, d, k, lib_built, monkeypatch):
         np.testing.assert_array_equal(ids, answers[3][0])
         np.testing.assert_array_equal(dd, answers[3][1])
     assert max(took[1:3]) < took[3] / 5, took
+
+
+@pytest.mark.parametrize("metric", [P.L2, P.MIPS])
+@pytest.mark.parametrize("n,nq,d,k", [(100_000, 20, 700, 20), (2000, 30_001, 8, 256)], ids=["segments", "chunks"])
+def test_more_than_one_segment_or_chunk(n, nq, d, k, metric, lib_built, monkeypatch):
+    """Point images past 128 MB (three segments, the candidate buffers carried over) and candidate buffers past 128 MB
+    (the queries in chunks)."""
+    both(random_points(np.float32, n, d, 1), random_points(np.float32, nq, d, 2), k, metric, monkeypatch)

@@ -103,3 +103,23 @@ def test_few_queries_with_growth(nq, lib_built):
     r = idx.search(q[-1:], 10, 40)  # a call after one that grew
     check(r, O.search("oracle", base, q[-1:], g, 10, 40))
     idx.close()
+
+
+@pytest.mark.parametrize("n", [1 << 23, (1 << 23) + 9], ids=["16-bit", "32-bit"])
+def test_widest_ids_of_4096_slots(n, lib_built):
+    """Ids that just fit 16-bit entries at 4,096 slots (23 bits), and ids that do not."""
+    rng = np.random.default_rng(6)
+    R = 12
+    base, q = random_points(np.uint8, n, 4, 7), random_points(np.uint8, 64, 4, 8)
+    g = np.empty((n, R + 1), np.uint32)
+    g[:, 0] = R
+    g[:, 1:] = rng.integers(0, n, (n, R), dtype=np.uint32)
+    idx = P.Index(base, R)
+    idx.set_graph(g)
+    o = O.search("oracle", base, q, g, 10, 60)
+    assert (o["ids"] > n // 2).any()
+    b = idx.batch(len(q), 10, 60, seen_slots=4096)
+    check(b.run(q, 10, 60), o)
+    b.close()
+    check(idx.search(q, 10, 60), o)
+    idx.close()

@@ -42,3 +42,24 @@ def test_thin_tiles(d, R, precision, lib_built):
                 want = P.point_distances(q, base, ids, metric)
                 np.testing.assert_array_equal(r.dists[live].view(np.uint32), want[live].view(np.uint32))
         idx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [1, 7, 9, 15, 17, 33, 95])
+@pytest.mark.parametrize("precision", [P.PREC_BF16, P.PREC_FP8])
+def test_padded_dimensions_add_nothing(d, precision, lib_built):
+    """Rows of any length score as the same rows with zeros up to a whole number of 16-byte chunks."""
+    n, R = 3000, 24
+    base, q = random_points(np.float32, n, d, d), random_points(np.float32, 200, d, d + 1)
+    g = O.random_graph(n, R, d + 2, min_deg=8)
+    pad = ((0, 0), (0, -d % 16))
+    for metric in (P.L2, P.MIPS):
+        got = []
+        for b, x in ((base, q), (np.pad(base, pad), np.pad(q, pad))):
+            idx = P.Index(b, R, metric)
+            idx.set_graph(g)
+            idx.set_precision(precision)
+            got.append(idx.search(x, 10, 40, precision=precision, parents=3))
+            idx.close()
+        for f in ("ids", "dists", "visited", "cmps"):
+            np.testing.assert_array_equal(getattr(got[0], f), getattr(got[1], f))
