@@ -1099,11 +1099,11 @@ int pann_search(pann_index* idx, const void* queries, uint32_t nq, const pann_qu
                       d_cmps, d_status, nullptr, 0, st, 0, 0, 0, 0, phase);
   };
   if (words <= 65536) {
-    // few queries seldom need the later tiers: they are launched only if the first one's counters ask for them. Saves
-    // 10 to 14 us where no hashset grows (100K x 128 uint8, beam 20: one query 128 -> 117 us, 32 queries 150 -> 139),
-    // costs 17 us where one does (a second wait, no emulation beside the first tier; beam 50: 508 -> 525). Of four sets
-    // none grew up to 8 queries, one at 16, two at 32, three at 64, where it no longer pays
-    const bool first_only = nq <= 32;
+    // few queries seldom need the later tiers: they are launched only if the first one's counters ask for them. Over 13
+    // built indexes that saves 64 queries 10 to 23 us where no hashset grows (30K x 100 int8, beam 10: 155 -> 140 us)
+    // and costs 17 us where one does (a second wait, no emulation beside the first tier; 100K x 128 uint8, beam 50:
+    // 510 -> 525, 128 queries 560 -> 577); past 64 queries most calls have one
+    const bool first_only = nq <= 64;
     std::vector<uint32_t> h(words + 16);
     rc = run(first_only ? TIERS_FIRST : TIERS_ALL);
     if (rc) return rc;
