@@ -115,9 +115,14 @@ constexpr uint64_t TC_WAIT_LIMIT = 1000000000ull;
 // float32 accuracy, and the Euclidean score is |b|^2 - 2 b.q + |q|^2 with the
 // row's squared norm precomputed (SearchArgs::lp_norms). The traversal, the
 // cutoff, the merge and the exact re-rank are those of the CUDA-core scoring.
-template <int MT, int PREC, bool TC>
-__global__ void __launch_bounds__(128, 6) search_tile_kernel(SearchArgs a, uint32_t W, uint32_t S, uint32_t CW,
-                                                          uint32_t CWs) {
+//
+// MINB: blocks an SM the registers are fitted to. 8 (64 registers) is the best for tiles whose state fills an SM's shared
+// memory with that many blocks or fewer, 12 (40 registers, 32 bytes spilled) where twelve fit and there are queries for
+// more than eight (bfloat16, 3,000 queries, one parent: 30K x 24, R 32, beam 45, 0.63 and 0.57 ms; 50K x 96, R 64, beam
+// 120, 2.33 and 2.51). Six blocks with point_dist in the re-rank spilled 80 bytes of 80 registers: 0.80 and 2.68 ms.
+template <int MT, int PREC, bool TC, int MINB>
+__global__ void __launch_bounds__(128, MINB) search_tile_kernel(SearchArgs a, uint32_t W, uint32_t S, uint32_t CW,
+                                                                uint32_t CWs) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -444,7 +449,13 @@ __global__ void __launch_bounds__(128, 6) search_tile_kernel(SearchArgs a, uint3
       } else {
         for (uint32_t i = tid; i < nr; i += blockDim.x) {
           const uint32_t id = key_id(fr[i]);
-          cand[i] = make_key(point_dist<DT_F32, MT>(a.points + (uint64_t)id * a.stride, qs, (int)a.d, (int)a.nchunks, 0), id);
+          // a chunk at a time: few rows of small tiles come here, and point_dist's twelve loads in flight made the
+          // whole kernel spill
+          const float4* row = reinterpret_cast<const float4*>(a.points + (uint64_t)id * a.stride);
+          const float4* q = reinterpret_cast<const float4*>(qs);
+          float r = 0.0f;
+          for (uint32_t c = 0; c < a.nchunks; c++) r = f32_chunk<MT>(r, __ldg(row + c), q[c]);
+          cand[i] = make_key(MT == MT_L2 ? r : -r, id);
         }
       }
     }
@@ -504,45 +515,53 @@ static int resident_blocks(const void* k, int threads, size_t smem) {
   return std::max(1, std::min({by_smem, by_regs, by_thr}));
 }
 
+// Blocks of 128 threads an SM holds of k. With tensor-core scoring the occupancy query has answered 1 even where 5 fit
+// (measured): then the blocks a multiprocessor holds by its shared memory, registers and threads, capped by tensor
+// memory (32 columns a block, 512 an SM).
+template <typename K>
+static int tile_occupancy(K k, size_t smem, bool tc) {
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 128, smem) != cudaSuccess || occ <= 0) occ = 1;
+  return tc ? std::min(std::max(occ, resident_blocks(reinterpret_cast<const void*>(k), 128, smem)), 16) : occ;
+}
+
 // Rows staged at once: the most that still gives the best occupancy among
 // CW, 3/4 CW and 1/2 CW (steps with more new candidates stage in rounds);
 // with tensor-core scoring, rounds of TC_ROWS rows.
 template <int MT, int PREC, bool TC>
 static int launch_tile_t(const pann_index* idx, const SearchArgs& a, uint32_t W, uint32_t S, uint32_t CW,
                          cudaStream_t st, uint32_t tile_rows) {
-  auto k = search_tile_kernel<MT, PREC, TC>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
-  if (e != cudaSuccess) return cuda_fail(e, "tile kernel attribute");
-  uint32_t CWs = TC ? TC_ROWS : CW;
-  size_t smem = tile_layout(idx->d, a.L, CW, S, idx->lp_stride, CWs, TC).total;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 128, smem) != cudaSuccess || occ <= 0) occ = 1;
-  if (!TC && tile_rows > 0) {
-    CWs = std::min<uint32_t>(CW, std::max<uint32_t>(16, (tile_rows + 15) & ~15u));
-    smem = tile_layout(idx->d, a.L, CW, S, idx->lp_stride, CWs).total;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 128, smem) != cudaSuccess || occ <= 0) occ = 1;
+  auto k = search_tile_kernel<MT, PREC, TC, 8>;
+  auto k12 = search_tile_kernel<MT, PREC, TC, 12>;
+  for (auto kern : {k, k12}) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr_max());
+    if (e != cudaSuccess) return cuda_fail(e, "tile kernel attribute");
   }
+  uint32_t CWs = TC ? TC_ROWS : CW;
+  if (!TC && tile_rows > 0) CWs = std::min<uint32_t>(CW, std::max<uint32_t>(16, (tile_rows + 15) & ~15u));
+  size_t smem = tile_layout(idx->d, a.L, CW, S, idx->lp_stride, CWs, TC).total;
+  int occ = tile_occupancy(k, smem, TC);
   for (uint32_t f = 3; f >= 2 && !TC && tile_rows == 0; f--) {
     const uint32_t cws = std::max<uint32_t>(32, (CW * f / 4 + 15) & ~15u);
     const size_t sm2 = tile_layout(idx->d, a.L, CW, S, idx->lp_stride, cws).total;
-    int occ2 = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k, 128, sm2) == cudaSuccess && occ2 > occ) {
+    const int occ2 = tile_occupancy(k, sm2, TC);
+    if (occ2 > occ) {
       occ = occ2;
       CWs = cws;
       smem = sm2;
     }
   }
-  if (TC) {
-    // the occupancy query has answered 1 block per SM for this kernel even
-    // where 5 fit (measured); the blocks a multiprocessor holds by its shared
-    // memory, registers and threads, capped by tensor memory: 32 columns a
-    // block, 512 an SM
-    occ = std::min(std::max(occ, resident_blocks(reinterpret_cast<const void*>(k), 128, smem)), 16);
+  if (a.nq > 8u * (uint32_t)idx->sm_count) {
+    const int occ12 = tile_occupancy(k12, smem, TC);
+    if (occ12 >= 12) {
+      k = k12;
+      occ = occ12;
+    }
   }
   const uint64_t want = a.nq;
   const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)occ * idx->sm_count));
   k<<<blocks, 128, smem, st>>>(a, W, S, CW, CWs);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "tile kernel launch");
   return PANN_OK;
 }
