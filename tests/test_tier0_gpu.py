@@ -123,3 +123,19 @@ def test_widest_ids_of_4096_slots(n, lib_built):
     b.close()
     check(idx.search(q, 10, 60), o)
     idx.close()
+
+
+def test_every_query_resident_where_narrow_entries_allow_it(lib_built):
+    """Few queries of long rows and beams: at 32-bit entries three of them fit on an SM, at 16 bits more; none of 500
+    waits for another to finish."""
+    n, d, R, nq = 1200, 3000, 32, 500
+    base, q = random_points(np.float32, n, d, 1), random_points(np.float32, nq, d, 2)
+    g = O.random_graph(n, R, 3, min_deg=24)
+    idx = P.Index(base, R)
+    idx.set_graph(g)
+    b = idx.batch(nq, 10, 600)
+    cfg = b.config()
+    b.close()
+    assert cfg["blocks"] * cfg["warps_per_block"] >= nq, cfg
+    check(idx.search(q, 10, 600), O.search("oracle", base, q, g, 10, 600))
+    idx.close()
