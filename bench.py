@@ -1052,6 +1052,27 @@ def run_reference(args):
     }
 
 
+# What a form's record has besides its rates: left out of the printed line.
+FORM_EXTRAS = {"scoring_error_vs_fp64", "reported_distances_equal_exact_f32", "recall_loss_at_plain_beam",
+               "stopped_early", "workload", "requests", "admission", "generate_seconds_host"}
+
+
+def printed(line: dict) -> dict:
+    """The line that goes to stdout: everything but the forms' sweeps and side figures (28 KB with them, more than a
+    reader of a process's last output gets). The whole record goes to stderr."""
+    def lean(v):
+        if isinstance(v, dict):
+            return {k: lean(x) for k, x in v.items()
+                    if k not in FORM_EXTRAS and not (isinstance(x, list) and len(x) > 4)}
+        return v
+
+    out = dict(line)
+    for key in ("details", "forms"):
+        if isinstance(out.get(key), dict):
+            out[key] = lean(out[key])
+    return out
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1076,7 +1097,8 @@ def main():
     args.warmup = max(args.warmup, 3)
     line = run_reference(args) if args.impl == "reference" else run_ours(args)
     if line is not None:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(printed(line)), flush=True)
 
 
 if __name__ == "__main__":
