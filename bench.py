@@ -1052,24 +1052,29 @@ def run_reference(args):
     }
 
 
-# What a form's record has besides its rates: left out of the printed line.
-FORM_EXTRAS = {"scoring_error_vs_fp64", "reported_distances_equal_exact_f32", "recall_loss_at_plain_beam",
-               "stopped_early", "workload", "requests", "admission", "generate_seconds_host"}
-
-
 def printed(line: dict) -> dict:
-    """The line that goes to stdout: everything but the forms' sweeps and side figures (28 KB with them, more than a
-    reader of a process's last output gets). The whole record goes to stderr."""
-    def lean(v):
-        if isinstance(v, dict):
-            return {k: lean(x) for k, x in v.items()
-                    if k not in FORM_EXTRAS and not (isinstance(x, list) and len(x) > 4)}
-        return v
+    """The line that goes to stdout: the contract's keys, the details without their sweep, and of each form its rate
+    (under the form's path in the record; of the precisions the best). The whole record, 28 KB with every form, goes to stderr: readers that keep
+    the last few KB of a process's output find the headline whole."""
+    rates = {}
 
-    out = dict(line)
-    for key in ("details", "forms"):
-        if isinstance(out.get(key), dict):
-            out[key] = lean(out[key])
+    def collect(path, v):
+        if isinstance(v, dict):
+            for key in ("qps_batched_graph", "qps_e2e", "qps", "capacity_qps_closed"):
+                if key in v:
+                    family, _, name = path.rpartition(".")
+                    at = family if name.startswith(("bf16", "fp8")) else path
+                    rates[at] = max(round(v[key]), rates.get(at, 0))
+                    return
+            for k, x in v.items():
+                collect(f"{path}.{k}" if path else k, x)
+
+    out = {k: v for k, v in line.items() if k not in ("forms", "build_roofline")}
+    if isinstance(out.get("details"), dict):
+        out["details"] = {k: v for k, v in out["details"].items() if not isinstance(v, list)}
+    if isinstance(line.get("forms"), dict):
+        collect("", line["forms"])
+        out["forms_qps"] = rates
     return out
 
 

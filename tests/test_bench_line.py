@@ -13,11 +13,11 @@ def test_printed_line_is_short_and_keeps_the_contract():
                 scoring_error_vs_fp64=dict(pairs=40000, abs_max=0.1))
     sweep = [dict(k=10, beam=b, recall=0.9, qps=1.0) for b in range(120)]
     line = dict(contract, details=dict(beam=45, recall_sweep=[[b, 0.9] for b in range(40)]),
-                forms=dict(precision_batched={f"form{i}": form for i in range(8)}, search_and_parse=dict(runs=sweep)))
+                forms=dict(precision_batched={f"bf16_{i}": dict(form, qps_batched_graph=i) for i in range(8)},
+                           range=dict(qps_e2e=10.4), search_and_parse=dict(runs=sweep)))
     out = bench.printed(line)
     assert {k: out[k] for k in contract} == contract
     assert out["details"] == dict(beam=45)
-    assert out["forms"]["precision_batched"]["form3"] == {k: form[k] for k in form if k != "scoring_error_vs_fp64"}
-    assert "runs" not in out["forms"]["search_and_parse"]
-    assert len(json.dumps(out)) < 4096 < len(json.dumps(line))
+    assert out["forms_qps"] == {"precision_batched": 7, "range": 10}
+    assert len(json.dumps(out)) < 2600 < len(json.dumps(line))
     assert line["details"]["recall_sweep"], "the record itself stays whole"
