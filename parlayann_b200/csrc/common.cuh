@@ -190,10 +190,12 @@ __device__ __forceinline__ uint64_t f32_chunk2(uint64_t r, float4 a, float4 b, f
 // query are zero-padded to whole 16-byte chunks; a padded term adds +0.0,
 // which leaves the running sum unchanged bit for bit (it starts at +0.0 and
 // can never be -0.0), so whole chunks are summed without per-element tests.
-// 16-byte chunks of a float row in flight at once: 12 of a 96-d row's 24
-// (the rest prefetched to L2) took the 1M x 96 build from 8.94 s to 8.12 s
-// (its prune steps score candidate rows this way), with the same graph; 24
-// slowed its searches (registers); the exact search itself was unchanged.
+// 16-byte chunks of a float row in flight at once, the rest of the row
+// prefetched to L2. Callers score a row a thread: pann_score, the quantized
+// search's re-rank, the emulation's start points and the build's rare prunes
+// sorted in global memory (searches and the other prunes go through
+// rowscore.cuh). 400K rows by score_kernel, 96 and 300 dimensions: 12
+// chunks 47 and 121 us, 4 chunks 47 and 128, 24 chunks 53 and 140.
 #ifndef PANN_F32_ROW_CHUNKS
 #define PANN_F32_ROW_CHUNKS 12
 #endif
@@ -217,10 +219,9 @@ __device__ __forceinline__ float dist_f32_row(const float4* __restrict__ row, co
 // Two rows against the same query, their loads and sums interleaved so the
 // two dependency chains overlap. rowB may be null (then db is not written).
 // Loads go in batches of PAIR_CHUNKS 16-byte chunks per row (the rows' other
-// lines are prefetched into L2 first), which keeps the register footprint
-// within the 168-register budget of three resident 128-thread blocks per SM
-// (the shared-memory seen tables allow three anyway); measured faster than
-// 4-chunk batches at four blocks and than 12- or 24-chunk batches, which spill.
+// lines are prefetched into L2 first). Callers: the range groundtruth (200
+// queries x 200K points, 96 and 300 dimensions: 8 chunks 4.66 and 7.60 ms, 4
+// chunks 4.72 and 8.15, 12 chunks 4.88 and 8.36) and the warp-a-query emulation.
 constexpr int PAIR_CHUNKS = 8;
 template <int DT, int MT, int CH = PAIR_CHUNKS>
 __device__ __forceinline__ void point_dist2(const uint8_t* __restrict__ rowA, const uint8_t* __restrict__ rowB,

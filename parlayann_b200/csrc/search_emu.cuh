@@ -687,7 +687,7 @@ __device__ __forceinline__ void emu_place_ranked_block(uint32_t* keys, uint32_t 
 // Block: emu_grow with every thread (the table state passed in, the
 // triggering key a). Returns false (every thread alike) if the grown table
 // does not fit `other_cap`; else *added = re-inserted keys and *a_seen =
-// whether a was found. ctl: 8 words of shared scratch.
+// whether a was found. ctl: 4 + nth / 32 words of shared scratch.
 __device__ __forceinline__ bool emu_grow_block(uint32_t* cur, uint32_t* other, uint32_t bits, uint32_t other_cap,
                                                uint32_t a, int tid, int nth, volatile uint32_t* ctl, uint32_t* added,
                                                bool* a_seen) {
